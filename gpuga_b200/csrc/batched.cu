@@ -35,6 +35,7 @@
 
 #include "engine.hpp"
 #include "exp_d.cuh"
+#include "fold.cuh"
 #include "powf_dd.cuh"
 
 namespace gpuga {
@@ -80,6 +81,7 @@ __global__ void decode_jobs(const JobView* __restrict__ jobs, const int2* __rest
   const JobView& J = jobs[jp.x];
   const int p = jp.y, nv = J.num_vars, Pstride = J.Pstride, potential_type = J.potential_type;
   const int num_types = J.num_types;
+  if (p == 0 && J.sp.count) *J.sp.count = 0;  // individuals left to the direct items this generation
   const float* __restrict__ pmin = J.pmin;
   const float* __restrict__ pmax = J.pmax;
   float* __restrict__ consts = J.consts;
@@ -271,8 +273,9 @@ __host__ __device__ __forceinline__ int pack_G(int G, bool staged, size_t fbytes
 // butterfly step form the same sum, so the result is deterministic, and every chain is
 // short (a sequential fold over 32/G atom slots per warp stalled the CTA).
 // GT: G as a compile-time constant (0: read from the item).
+// p: the individual of this lane (lanes below G; -1: none).
 template <int GT>
-__device__ __forceinline__ void fold_item(const WorkItem& it, int P, int Nc, const double* red,
+__device__ __forceinline__ void fold_item(const WorkItem& it, int p, int Nc, const double* red,
                                           double* __restrict__ res) {
   __syncthreads();
   const int G = GT ? GT : item_G(it), nw = blockDim.x >> 5;
@@ -281,20 +284,19 @@ __device__ __forceinline__ void fold_item(const WorkItem& it, int P, int Nc, con
     double s = 0.0;
     for (int w = 0; w < nw; ++w) s += red[(size_t)k * blockDim.x + w * 32 + lane];
     for (int o = G; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    const int p = it.p0 + lane;
-    if (lane < G && p < P) res[((size_t)p * Nc + it.config) * kResK + k] = s;
+    if (lane < G && p >= 0) res[((size_t)p * Nc + it.config) * kResK + k] = s;
   }
 }
 
 // Same for partial sums held in registers (they are first written out).
 template <int GT>
-__device__ __forceinline__ void reduce_item(const WorkItem& it, int P, int Nc, double (&acc)[kResK],
+__device__ __forceinline__ void reduce_item(const WorkItem& it, int p, int Nc, double (&acc)[kResK],
                                             unsigned char* smem, double* __restrict__ res) {
   __syncthreads();
   double* red = reinterpret_cast<double*>(smem);
 #pragma unroll
   for (int k = 0; k < kResK; ++k) red[(size_t)k * blockDim.x + threadIdx.x] = acc[k];
-  fold_item<GT>(it, P, Nc, red, res);
+  fold_item<GT>(it, p, Nc, red, res);
 }
 
 // Geometry of one configuration as a CTA sees it.  Unstaged: the global CSR
@@ -717,7 +719,7 @@ __device__ __forceinline__ void tersoff_item(const JobView* __restrict__ jobs, c
   }
   if (!FORCE) {
     red[7 * BLK + threadIdx.x] = 0.0;
-    fold_item<GT>(it, P, S.Nc, red, res);
+    fold_item<GT>(it, it.p0 + lane < P ? it.p0 + lane : -1, S.Nc, red, res);
     return;
   }
   __syncthreads();
@@ -768,7 +770,7 @@ __device__ __forceinline__ void tersoff_item(const JobView* __restrict__ jobs, c
 #pragma unroll
     for (int k = 0; k < 7; ++k) red[k * BLK + threadIdx.x] = 0.0;
     red[7 * BLK + threadIdx.x] = ferr;
-    fold_item<GT>(it, P, S.Nc, red, res);
+    fold_item<GT>(it, it.p0 + lane < P ? it.p0 + lane : -1, S.Nc, red, res);
     return;
   }
   auto replay = [&](const double* ftab) {
@@ -825,82 +827,6 @@ __device__ __forceinline__ void tersoff_item(const JobView* __restrict__ jobs, c
     }
     __syncthreads();
     replay(ftab);
-  }
-}
-
-// fitness.cu:329-331, 437-555 in FP64 for individual p, by one warp: lane c sums configurations
-// c, c + 32, ... in order, then a butterfly; the same order whichever warp or launch folds, and
-// the same operations: every product and sum is an explicit intrinsic, so that the compiler's
-// choice of contracting a * b + c into an FMA cannot differ between the kernels this is inlined in.
-// Reads go through L2 (ld.cg): other CTAs of the same launch wrote the results.
-__device__ __forceinline__ void fold_fitness(const JobView& J, int p, int lane) {
-  const int Nc = J.v.Nc, Nc_force = J.Nc_force;
-  const double* __restrict__ res = J.res;
-  const double* __restrict__ E_ref = J.E_ref;
-  const double* __restrict__ W_ref = J.W_ref;
-  double eE = 0, eW = 0, eF = 0;
-  for (int c = lane; c < Nc; c += 32) {
-    const double* r = res + ((size_t)p * Nc + c) * kResK;
-    if (c >= Nc_force) {
-      const double de = __ldcg(r) - E_ref[c];
-      eE = __fma_rn(de, de, eE);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const double dw = __ldcg(r + 1 + k) - W_ref[c + (size_t)Nc * k];
-        eW = __fma_rn(dw, dw, eW);
-      }
-    } else {
-      eF += __ldcg(r + 7);
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    eE += __shfl_xor_sync(0xffffffffu, eE, o);
-    eW += __shfl_xor_sync(0xffffffffu, eW, o);
-    eF += __shfl_xor_sync(0xffffffffu, eF, o);
-  }
-  if (lane == 0) {
-    const double rE = sqrt(eE / J.nE), rW = sqrt(eW / J.nW), rF = sqrt(eF / J.nF);
-    J.fitness[p] = __dadd_rn(__dadd_rn(__dmul_rn((double)J.wE, rE), __dmul_rn((double)J.wW, rW)),
-                             __dmul_rn((double)J.wF, rF));
-    if (J.comps) {
-      J.comps[3 * (size_t)p + 0] = rE;
-      J.comps[3 * (size_t)p + 1] = rW;
-      J.comps[3 * (size_t)p + 2] = rF;
-    }
-  }
-}
-
-// End of every work item: its results for individuals p0 .. p0 + G - 1 are written.  Each of those
-// individuals' completion count goes up by one with a release-acquire atomic (the CTA barrier
-// orders every thread's writes before it, and release is cumulative); the item that brings an individual to Nc
-// configurations folds its fitness and resets the count for the next generation.  Nothing waits.
-// Release-acquire increment at device scope: releases the CTA's writes ordered before it (by the
-// preceding CTA barrier) and acquires the writes released by earlier increments.
-__device__ __forceinline__ int atomic_add_acq_rel(int* a, int v) {
-  int old;
-  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], %2;" : "=r"(old) : "l"(a), "r"(v) : "memory");
-  return old;
-}
-
-__device__ __forceinline__ void finish_item(const JobView* __restrict__ jobs, const WorkItem& it, int G) {
-  const JobView& J = jobs[it.job];
-  if (!J.fit_count) return;
-  __shared__ int s_last[32];
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    const int p = it.p0 + threadIdx.x;
-    int last = 0;
-    if (threadIdx.x < G && p < J.P) last = atomic_add_acq_rel(&J.fit_count[p], 1) == J.v.Nc - 1;
-    s_last[threadIdx.x] = last;
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  for (int g = threadIdx.x >> 5; g < G; g += blockDim.x >> 5) {
-    if (!s_last[g]) continue;  // warp-uniform
-    __threadfence();
-    fold_fitness(J, it.p0 + g, lane);
-    if (lane == 0) J.fit_count[it.p0 + g] = 0;
   }
 }
 
@@ -1175,18 +1101,29 @@ __device__ __forceinline__ void nn_pairs(const float* __restrict__ wsm, int lane
   for (int u = 0; u < NP; ++u) p2[u] = with_p2 ? (float)(p2d[u] - (double)b2) : 0.f;
 }
 
+// Individual of slot `slot` of a pair item: the population's own order, or, for a job with a pair
+// expansion (spectral.cu), the list of the individuals that it left to the direct items; limit: how
+// many there are.
+__device__ __forceinline__ int pair_individual(const JobView& J, int slot, int limit) {
+  if (slot >= limit) return -1;
+  return J.sp.list ? __ldcg(J.sp.list + slot) : slot;
+}
+
 template <int KIND, int NMAX, bool FORCE>
-__device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, const WorkItem& it, unsigned char* smem) {
+__device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, const WorkItem& it, int limit,
+                                          unsigned char* smem) {
   const JobView& J = jobs[it.job];
   const DevView S = J.v;
-  const int P = J.P, Pstride = J.Pstride, nn = J.num_neurons, nv = J.num_vars;
+  const int Pstride = J.Pstride, nn = J.num_neurons, nv = J.num_vars;
   const NNTaper tp = J.tp;
   const float* __restrict__ weights = J.weights;
   double* __restrict__ res = J.res;
   float* __restrict__ fdump = J.fdump;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int p = it.p0 + lane;
-  const int pl = p < P ? p : it.p0;
+  // lane -> individual (-1: none); lanes without one compute the group's first again
+  const int p = pair_individual(J, it.p0 + lane, limit);
+  const int p_first = pair_individual(J, it.p0, limit);
+  const int pl = p >= 0 ? p : p_first;
   const Consts kc{J.consts, Pstride, pl};
   RIC R;
   if (KIND == 1) load_ri(kc, R);
@@ -1196,8 +1133,8 @@ __device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, cons
     __syncthreads();
     for (int t = threadIdx.x; t < nv * 32; t += blockDim.x) {
       const int m = t >> 5, l = t & 31;
-      const int pp = it.p0 + l < P ? it.p0 + l : it.p0;
-      wsm[NNSmem<NMAX>::offset(m, nn, l)] = weights[(size_t)m * Pstride + pp];
+      const int pp = pair_individual(J, it.p0 + l, limit);
+      wsm[NNSmem<NMAX>::offset(m, nn, l)] = weights[(size_t)m * Pstride + (pp >= 0 ? pp : p_first)];
     }
     __syncthreads();
   }
@@ -1266,7 +1203,7 @@ __device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, cons
       const double dy = F[1] - (double)S.force_ref[i + N];
       const double dz = F[2] - (double)S.force_ref[i + 2 * (size_t)N];
       acc[7] += dx * dx + dy * dy + dz * dz;
-      if (fdump && p < P) {
+      if (fdump && p >= 0) {
         const int Nf = S.N_force;
         fdump[((size_t)p * 3 + 0) * Nf + i] = (float)F[0];
         fdump[((size_t)p * 3 + 1) * Nf + i] = (float)F[1];
@@ -1449,7 +1386,7 @@ __device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, cons
       finish_atom(0, ks);
     }
   }
-  reduce_item<32>(it, P, S.Nc, acc, smem, res);  // pair items hold 32 individuals
+  reduce_item<32>(it, p, S.Nc, acc, smem, res);  // pair items hold 32 individuals
 }
 
 // RI: three CTAs per SM (at most 85 registers); NN2B: two (128 registers, two pairs per weight
@@ -1458,16 +1395,25 @@ __device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, cons
 // launch; the rigid ion's go in two launches of single-kind instantiations (job_items).
 // ONLY: 0 both kinds of items (item_force), 1 force items only, 2 energy/virial items only (one
 // body, so its own register allocation).
+// A job with a pair expansion has items here for the individuals that the expansion could not
+// represent, usually none: its items beyond their number return at once, and where every job of the
+// launch has one the grid is no larger than the GPU holds, each CTA walking the items at its stride.
 template <int KIND, int NMAX, int ONLY>
 __global__ void __launch_bounds__(kBlock, KIND == 1 ? 3 : 2) pair_batched(const JobView* __restrict__ jobs,
-                                                                         const WorkItem* __restrict__ items) {
+                                                                         const WorkItem* __restrict__ items, int count) {
   extern __shared__ __align__(16) unsigned char smem[];
-  const WorkItem it = items[blockIdx.x];
-  if (ONLY == 1 || (ONLY == 0 && item_force(it)))
-    pair_item<KIND, NMAX, true>(jobs, it, smem);
-  else
-    pair_item<KIND, NMAX, false>(jobs, it, smem);
-  finish_item(jobs, it, 32);
+  for (int b = blockIdx.x; b < count; b += gridDim.x) {
+    const WorkItem it = items[b];
+    const JobView& J = jobs[it.job];
+    const int limit = J.sp.list ? __ldcg(J.sp.count) : J.P;
+    if (it.p0 >= limit) continue;
+    if (b != (int)blockIdx.x) __syncthreads();  // the previous item's reads of shared memory
+    if (ONLY == 1 || (ONLY == 0 && item_force(it)))
+      pair_item<KIND, NMAX, true>(jobs, it, limit, smem);
+    else
+      pair_item<KIND, NMAX, false>(jobs, it, limit, smem);
+    finish_individuals(J, threadIdx.x < 32 ? pair_individual(J, it.p0 + (int)threadIdx.x, limit) : -1, 32);
+  }
 }
 
 // --------------------------------------------------------------------------- fitness
@@ -1576,6 +1522,7 @@ JobView make_job_view(const Engine* e, const Plan* plan) {
   j.fitness = plan->d_fitness;
   j.comps = plan->d_comps;
   j.fit_count = plan->d_fitcnt;
+  j.sp = plan->sp;
   return j;
 }
 
@@ -1584,6 +1531,7 @@ LaunchSet::~LaunchSet() {
   if (h_jobs) cudaFreeHost(h_jobs);
   if (d_items) cudaFree(d_items);
   if (d_indmap) cudaFree(d_indmap);
+  if (d_specmap) cudaFree(d_specmap);
   if (side) cudaStreamDestroy(side);
   if (fork) cudaEventDestroy(fork);
   if (join) cudaEventDestroy(join);
@@ -1602,9 +1550,10 @@ struct ItemSpec {
   double cost, units, flops, sfu;
 };
 struct LaunchKey {
-  int kind, zclass, nmax, force, lo;
+  int kind, zclass, nmax, force, lo, expansion;
   bool operator<(const LaunchKey& o) const {
-    return std::tie(kind, zclass, nmax, force, lo) < std::tie(o.kind, o.zclass, o.nmax, o.force, o.lo);
+    return std::tie(kind, zclass, nmax, force, lo, expansion) <
+           std::tie(o.kind, o.zclass, o.nmax, o.force, o.lo, o.expansion);
   }
 };
 // A plan's work items grouped by launch (job index 0), with their shared-memory and global-scratch needs.
@@ -1771,7 +1720,7 @@ int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<I
     // force and energy/virial items share a launch, except the rigid ion's: its two bodies under
     // one register allocation spilled more and ran 3 % slower than two single-kind kernels on two
     // streams (300-configuration set: 5.92 vs 5.74 ms per generation)
-    const LaunchKey key{kind, zc, nmax, kind == 1 && force ? 1 : 0, lo ? 1 : 0};
+    const LaunchKey key{kind, zc, nmax, kind == 1 && force ? 1 : 0, lo ? 1 : 0, 0};
     smem_need[key] = std::max(smem_need[key], smem);
     double cf = 0, cs = 0;
     const bool half = kind != 0 && (!force || once);  // unordered pairs evaluated once
@@ -1795,6 +1744,24 @@ int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<I
           {WorkItem{c, p0, pack_G(G, staged, fbytes, global, Grule, force, once), job, gofs}, cf * cnt, (double)Na * cnt, cf * cnt, cs * cnt});
     }
   }
+  if (d.sp.M) {
+    // the pair expansion's items: a force configuration, or up to kSpecEvBlocks energy/virial ones, x 32
+    // individuals; the direct items above then take only the individuals that it leaves to them
+    // (pair_batched)
+    const LaunchKey key{kind, 0, 0, 0, 0, 1};
+    smem_need[key] = 0;
+    for (int c = 0; c < ts.Nc; c += c < ts.Nc_force ? 1 : kSpecEvBlocks) {
+      const bool force = c < ts.Nc_force;
+      const int nev = force ? 0 : std::min(kSpecEvBlocks, ts.Nc - c);
+      double units = 0;
+      for (int k = c; k < c + (force ? 1 : nev); ++k) units += ts.Na[k];
+      const double products = force ? e->h_spec_blocks[c] : (double)nev * d.sp.ncb;
+      for (int p0 = 0; p0 < P; p0 += 32) {
+        const double cnt = std::min(32, P - p0), fl = 128.0 * products * cnt;
+        groups[key].push_back({WorkItem{c, p0, pack_G(32, false, 0, false, 32, force), job, nev}, fl, units * cnt, fl, 0.0});
+      }
+    }
+  }
   return GPUGA_OK;
 }
 
@@ -1806,9 +1773,13 @@ int set_smem(K kernel) {
 
 // configure_only: raise the dynamic shared-memory limit of the launch's kernel
 // (done when a launch set is built, never inside a stream capture).
+constexpr int kFallbackGrid = 2 * 148;  // two CTAs per SM walk the direct items of jobs with a pair expansion
+
 int launch_one(const LaunchSet* ls, const Launch& L, cudaStream_t st, bool configure_only) {
   const dim3 grid(L.count), block(kBlock);
+  const dim3 pgrid(L.fallback ? std::min(L.count, kFallbackGrid) : L.count);
   const WorkItem* items = ls->d_items + L.first;
+  if (L.expansion) return configure_only ? GPUGA_OK : spectral_items_launch(ls->d_jobs, items, L.count, st);
 #define GPUGA_TERSOFF1(ZC, NT)                                                          \
   do {                                                                                  \
     if (configure_only) {                                                               \
@@ -1831,7 +1802,7 @@ int launch_one(const LaunchSet* ls, const Launch& L, cudaStream_t st, bool confi
       GPUGA_TRY(set_smem(pair_batched<KD, NM, ON>));                                  \
       break;                                                                          \
     }                                                                                 \
-    pair_batched<KD, NM, ON><<<grid, block, L.smem, st>>>(ls->d_jobs, items);         \
+    pair_batched<KD, NM, ON><<<pgrid, block, L.smem, st>>>(ls->d_jobs, items, L.count); \
   } while (0)
 #define GPUGA_PAIR(KD, NM) GPUGA_PAIR1(KD, NM, 0)
   if (L.kind == 0) {
@@ -1863,8 +1834,9 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
                     const std::vector<std::pair<const float*, double*>>* targets, const std::vector<char>* only) {
   std::map<LaunchKey, std::vector<ItemSpec>> groups;
   std::map<LaunchKey, size_t> smem_need;
-  std::vector<int2> indmap;
+  std::vector<int2> indmap, specmap, by_class[5];
   ls->jobs.clear();
+  bool plain_pairs[3] = {false, false, false};  // some job of the kind evaluates every pair directly
   for (size_t j = 0; j < jobs.size(); ++j) {
     Engine* e = jobs[j].first;
     Plan* plan = jobs[j].second;
@@ -1904,6 +1876,11 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
       ls->jobs.back().fitness = (*targets)[j].second;
     }
     for (int p = 0; p < jobs[j].second->P; ++p) indmap.push_back(make_int2((int)j, p));
+    if (plan->sp.M) {
+      for (int p = 0; p < plan->P; ++p) by_class[spectral_class(e->d)].push_back(make_int2((int)j, p));
+    } else if (e->d.potential_type != 1 && e->d.potential_type != 2) {
+      plain_pairs[is_ri_type(e->d.potential_type) ? 1 : 2] = true;
+    }
   }
   std::vector<WorkItem> all;
   ls->launches.clear();
@@ -1915,6 +1892,8 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
     L.zclass = kv.first.zclass;
     L.nmax = kv.first.nmax;
     L.lo = kv.first.lo != 0;
+    L.expansion = kv.first.expansion != 0;
+    L.fallback = L.kind != 0 && !L.expansion && !plain_pairs[L.kind];
     int nforce = 0;
     for (auto& t : v) nforce += item_force(t.w) ? 1 : 0;
     L.force = nforce == 0 ? 0 : (nforce == (int)v.size() ? 1 : 2);
@@ -1929,9 +1908,11 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
     }
     ls->launches.push_back(L);
   }
-  // longest launches first so that the side stream starts the big ones early
-  std::stable_sort(ls->launches.begin(), ls->launches.end(),
-                   [](const Launch& a, const Launch& b) { return a.flops > b.flops; });
+  // longest launches first so that the side stream starts the big ones early; the direct items of
+  // jobs with a pair expansion usually have nothing to do
+  std::stable_sort(ls->launches.begin(), ls->launches.end(), [](const Launch& a, const Launch& b) {
+    return a.fallback != b.fallback ? b.fallback : a.flops > b.flops;
+  });
   ls->total_individuals = (int)indmap.size();
   // where the fitness is folded (gpuga_options.fitness_fold; a partial set never folds in its items).
   // The fold launch is the default: the count's round trip at the end of every item holds the
@@ -1945,6 +1926,15 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
   GPUGA_CUDA(cudaMemcpy(ls->d_items, all.data(), sizeof(WorkItem) * all.size(), cudaMemcpyHostToDevice));
   GPUGA_CUDA(cudaMalloc(&ls->d_indmap, sizeof(int2) * std::max<size_t>(indmap.size(), 1)));
   GPUGA_CUDA(cudaMemcpy(ls->d_indmap, indmap.data(), sizeof(int2) * indmap.size(), cudaMemcpyHostToDevice));
+  for (int k = 0; k < 5; ++k) {
+    ls->spec_class[k] = (int)by_class[k].size();
+    specmap.insert(specmap.end(), by_class[k].begin(), by_class[k].end());
+  }
+  ls->spec_individuals = (int)specmap.size();
+  if (!specmap.empty()) {
+    GPUGA_CUDA(cudaMalloc(&ls->d_specmap, sizeof(int2) * specmap.size()));
+    GPUGA_CUDA(cudaMemcpy(ls->d_specmap, specmap.data(), sizeof(int2) * specmap.size(), cudaMemcpyHostToDevice));
+  }
   GPUGA_CUDA(cudaMalloc(&ls->d_jobs, sizeof(JobView) * std::max<size_t>(ls->jobs.size(), 1)));
   GPUGA_CUDA(cudaMallocHost(&ls->h_jobs, sizeof(JobView) * std::max<size_t>(ls->jobs.size(), 1)));
   GPUGA_CUDA(cudaMemcpy(ls->d_jobs, ls->jobs.data(), sizeof(JobView) * ls->jobs.size(), cudaMemcpyHostToDevice));
@@ -1994,6 +1984,7 @@ int launchset_enqueue(LaunchSet* ls, cudaStream_t st) {
   const int total = ls->total_individuals;
   decode_jobs<<<(total + 127) / 128, 128, 0, st>>>(ls->d_jobs, ls->d_indmap, total);
   GPUGA_CUDA(cudaGetLastError());
+  if (ls->spec_individuals > 0) GPUGA_TRY(spectral_coefficients(ls, st));
   // several launches (job mixes with several kernel classes): every second one on the side stream
   const bool any_side = ls->launches.size() > 1 && !ls->timing;
   if (any_side) {
@@ -2003,7 +1994,7 @@ int launchset_enqueue(LaunchSet* ls, cudaStream_t st) {
   GPUGA_TRY(launchset_collect_timing(ls));
   for (size_t k = 0; k < ls->launches.size(); ++k) {
     const Launch& L = ls->launches[k];
-    cudaStream_t s = (k & 1) && any_side ? ls->side : st;
+    cudaStream_t s = any_side && ((k & 1) || L.fallback) ? ls->side : st;
     if (ls->timing) GPUGA_CUDA(cudaEventRecord(ls->tev[2 * k], s));
     GPUGA_TRY(launch_one(ls, L, s, false));
     if (ls->timing) GPUGA_CUDA(cudaEventRecord(ls->tev[2 * k + 1], s));
@@ -2109,6 +2100,7 @@ int plan_build(Engine* e, int P, Plan** out) {
   GPUGA_TRY(e->alloc(&plan->d_fitness, (size_t)P));
   GPUGA_TRY(e->alloc(&plan->d_comps, (size_t)3 * P));
   GPUGA_TRY(e->alloc(&plan->d_fitcnt, (size_t)P));
+  if (d.sp.M) GPUGA_TRY(spectral_plan(e, plan.get()));
   GPUGA_CUDA(cudaMemset(plan->d_fitcnt, 0, sizeof(int) * (size_t)P));
   GPUGA_TRY(e->alloc(&plan->d_pop, (size_t)P * d.num_vars));
   GPUGA_CUDA(cudaMallocHost(&plan->h_pop, sizeof(float) * (size_t)P * d.num_vars));

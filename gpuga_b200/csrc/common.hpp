@@ -41,6 +41,7 @@ struct PotentialSpec {
   std::vector<float> pmin, pmax;
   float nn_r1 = 7.0f, nn_r2 = 8.0f;  // nn2b.cuh:36-37
   int nn_consistent = 0;              // 0 keeps nn2b.cu:147-148 order
+  size_t expansion_bytes = 16ull << 30;  // most device memory for the pair expansion's moments
   int ri_self = 0;                    // RI: subtract the damped-Coulomb self energy (off in ri.cu)
 };
 

@@ -40,7 +40,42 @@ constexpr int kRiCfgLin = 66;         // RI linear energy/virial sums per config
 // z neighbors (0: beyond the supported 16).
 inline int tersoff_zclass(int z) { return z <= 4 ? 4 : (z <= 8 ? 8 : (z <= 16 ? 16 : 0)); }
 
+// The pair expansion of a rigid-ion or NN2B training set (spectral.cu): the distance range of each
+// pair type in pieces, on each of which the pair energy is a Chebyshev series.
+constexpr int kSpecMaxPieces = 32;
+constexpr int kSpecMaxK = 96;         // terms of a piece (a multiple of 8)
+constexpr int kSpecMaxCols = 1024;    // columns of all pieces and of the linear terms
+constexpr int kSpecEvBlocks = 12;     // energy/virial configurations per work item
+constexpr int kSpecWarps = 4;
+struct SpecPiece {
+  double mid, half;  // x = (d - mid) / half
+  double to;         // the piece holds the pairs of its type with d < to (and not in an earlier piece)
+  int type;          // pair type (0 for NN2B)
+  int K, node0;      // terms (a multiple of 8), first node
+  int ctab;          // first entry of cos(pi j / (2K)), j < 4K, in SpecView::ctab
+  int cb[kSpecMaxK / 8];  // column block of its terms 8 b .. 8 b + 7
+};
+struct SpecView {
+  const SpecPiece* pieces;
+  int n_pieces, n_nodes;    // n_nodes = sum of K
+  int ncb, n_lin;           // column blocks of 8: the n_lin linear columns first, then the pieces' terms by degree
+  int n_items;              // work items per group of individuals
+  int n_part;               // rows of `part`
+  const double* ctab;
+  const double* M;          // [row block][column block][8 x 8]
+  const int* row_block;     // [Nc_force + 1] first row block of each force configuration; then the energy/virial blocks
+  // per plan
+  double* coef;             // [individuals / 8][column block][8 x 8]
+  uint8_t* need;            // [piece][Pstride] column blocks in use
+  double* part;             // [n_part][Pstride]: squared errors per force configuration, then of the energies
+                            // and of the virials per energy/virial item
+  int* flagged;             // [P] 1: left to the direct items
+  int* list;                // flagged individuals, *count of them
+  int* count;
+};
+
 struct DevSet {
+  SpecView sp{};               // sp.M == nullptr: every pair is evaluated directly
   int Nc = 0, Nc_force = 0, N = 0, N_force = 0, B = 0, max_Na = 0, max_Z = 0;
   int potential_type = -1, num_types = 1, num_neurons = 0, num_vars = 0;
   int* Na = nullptr;
@@ -163,10 +198,13 @@ struct JobView {
   int* fit_count;        // [P] configurations of this generation finished per individual; the work
                          // item that finishes an individual's last one folds its fitness (reset to
                          // 0 there).  Null: a partial launch set (no fold).
+  SpecView sp;           // sp.M == nullptr: no pair expansion
 };
 
 struct Launch {
   int kind = 0;        // 0 Tersoff, 1 RI, 2 NN2B
+  bool expansion = false;  // RI / NN2B items of the pair expansion (spectral.cu)
+  bool fallback = false;   // RI / NN2B direct items that only take the individuals the expansion left
   int zclass = 4;      // Tersoff register-array size
   int nmax = 0;        // NN2B register-array size; Tersoff: number of atom types
   int force = 0;       // the launch's items: 0 energy/virial, 1 force (gather pass), 2 both
@@ -188,6 +226,9 @@ struct LaunchSet {
   WorkItem* d_items = nullptr;
   int2* d_indmap = nullptr;    // global individual -> (job, p)
   int total_individuals = 0;
+  int2* d_specmap = nullptr;   // the individuals of jobs with a pair expansion -> (job, p), by kernel class
+  int spec_class[5] = {0, 0, 0, 0, 0};  // how many of each (spectral_class)
+  int spec_individuals = 0;
   bool folds = true;           // the items fold every individual's fitness (no fitness_jobs launch)
   cudaStream_t side = nullptr;
   cudaEvent_t fork = nullptr, join = nullptr;
@@ -224,6 +265,7 @@ struct Plan {
   double* d_res = nullptr;     // [P][Nc][kResK]
   double* d_fitness = nullptr; // [P]
   double* d_comps = nullptr;   // [P][3]
+  SpecView sp{};               // pair expansion: the training set's view with this plan's buffers
   int* d_fitcnt = nullptr;     // [P] per-generation completion counts (JobView::fit_count)
   float* d_pop = nullptr;      // [P][d] staging
   float* h_pop = nullptr;      // pinned
@@ -250,6 +292,7 @@ struct Engine {
   float* d_pmin = nullptr;
   float* d_pmax = nullptr;
   std::vector<int> h_NN, h_off, h_nbr, h_zmax;  // host copies of the neighbor list
+  std::vector<int> h_spec_blocks;               // pair expansion: 8 x 8 products per force configuration
   std::vector<char> h_pair_sym;                 // NN2B: per configuration, bond list symmetric
   std::map<int, std::unique_ptr<Plan>> plans;    // keyed by population size
   size_t device_bytes = 0;
@@ -276,6 +319,15 @@ struct Engine {
     return dalloc(reinterpret_cast<void**>(p), n * sizeof(T));
   }
 };
+
+// spectral.cu
+int spectral_build(Engine* e);                 // moments of the training set (where the expansion pays)
+int spectral_plan(Engine* e, Plan* plan);      // per-population buffers
+size_t spectral_bytes(const PotentialSpec& spec, const TrainingSet& ts);  // estimate
+int spectral_class(const DevSet& d);           // 0 rigid ion, 1-4 network width classes
+// Coefficients of every individual of the set, then (per launch) the items.
+int spectral_coefficients(const LaunchSet* ls, cudaStream_t st);
+int spectral_items_launch(const JobView* jobs, const WorkItem* items, int count, cudaStream_t st);
 
 // geometry.cu
 int build_geometry(Engine* e);

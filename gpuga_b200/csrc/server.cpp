@@ -109,6 +109,11 @@ size_t estimate_bytes(const PotentialSpec& spec, const TrainingSet& ts, int P) {
   double bytes = 64.0 * ts.N + 88.0 * bonds + (tersoff ? 4.0 * trip : 0.0);
   bytes += (double)P * ts.Nc * kResK * 8.0 + (double)P * (spec.num_vars + 40) * 8.0;
   if (spec.type == 3) bytes += 4.0 * P * force_bonds;  // NN2B force items' per-pair scratch
+  if (spec.expansion_bytes) {
+    // pair expansion: moments, at most what the engine allows, and coefficients
+    const double m = (double)spectral_bytes(spec, ts);
+    bytes += std::min(m, (double)spec.expansion_bytes) + (m > 0 ? (double)P * kSpecMaxCols * 8.0 : 0.0);
+  }
   return (size_t)(1.25 * bytes) + (8u << 20);
 }
 
@@ -503,6 +508,10 @@ int gpuga_server_submit(gpuga_server* s, const char* dir, unsigned seed, int gen
   j->gens_total = generations > 0 ? generations : j->gp.maximum_generation;
   if (generations > 0 && j->gp.maximum_generation < generations) j->gp.maximum_generation = generations;
   j->bytes = estimate_bytes(j->spec, j->ts, j->gp.population_size);
+  if ((double)j->bytes > s->budget && j->spec.expansion_bytes) {
+    j->spec.expansion_bytes = 0;  // without the moments it may fit: every pair evaluated directly
+    j->bytes = estimate_bytes(j->spec, j->ts, j->gp.population_size);
+  }
   return enqueue_job(s, std::move(j), job_id);
 }
 
@@ -526,7 +535,9 @@ int gpuga_server_submit_engine(gpuga_server* s, gpuga_engine* e, int population_
   j->gp.maximum_generation = generations;
   j->gens_total = generations;
   j->bytes = (size_t)((double)population_size * e->e->d.Nc * kResK * 8.0 +
-                      (double)population_size * (e->e->d.num_vars + 40) * 8.0) + (1u << 20);
+                      (double)population_size * (e->e->d.num_vars + 40) * 8.0 +
+                      (e->e->d.sp.M ? (double)population_size * (e->e->d.sp.ncb * 8.0 + e->e->d.sp.n_part) * 8.0
+                                    : 0.0)) + (1u << 20);
   return enqueue_job(s, std::move(j), job_id);
 }
 

@@ -146,10 +146,13 @@ int gpuga_batched_forces(gpuga_engine* e, int P, const float* pop01, float* forc
  * per_launch (may be NULL) receives up to `cap` rows of 8 doubles:
  * {kind (0 Tersoff, 1 RI, 2 NN2B), register class, items (0 energy/virial, 1 force, 2 both), CTAs,
  *  (individual, atom) units, algorithmic FP32 flops, transcendental calls, mean device ms per
- *  generation while timing is on}. */
+ *  generation while timing is on}.  A rigid-ion or NN2B set evaluated through its pair expansion has one
+ * launch of matrix products (class 0, FP64 flops) and the launches of the direct items, which then only take
+ * the individuals that the expansion does not represent. */
 int gpuga_plan_info(gpuga_engine* e, int P, int* n_launches, double* per_launch, int cap);
 /* Kernel launches per generation of the batched path for population size P: the decode, the item
- * launches and, when the items do not fold the fitness (gpuga_options.fitness_fold), the fold. */
+ * launches, the coefficients of pair expansions and, when the items do not fold the fitness
+ * (gpuga_options.fitness_fold), the fold. */
 int gpuga_plan_kernels(gpuga_engine* e, int P, int* kernels);
 /* The force-item tile of every configuration (tiles[Nc], gpuga_options.tiles codes 1-5; 0 for
  * energy/virial and non-Tersoff configurations) of the plan for population size P, and the host time
