@@ -285,8 +285,8 @@ int gpuga_plan_kernels(gpuga_engine* h, int P, int* kernels) {
   int s = plan_get(h->e, P, &plan);
   if (s != GPUGA_OK) return s;
   const LaunchSet* ls = plan->ls.get();
-  // decode (+ pair coefficients) + items (+ fitness fold)
-  *kernels = 1 + (int)ls->launches.size() + (ls->folds ? 0 : 1);
+  // decode and pair coefficients, items (+ fitness fold)
+  *kernels = (ls->total_individuals > ls->spec_individuals) + (int)ls->launches.size() + (ls->folds ? 0 : 1);
   for (int n : ls->spec_class) *kernels += n > 0;
   return GPUGA_OK;
 }

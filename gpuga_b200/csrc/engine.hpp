@@ -42,11 +42,10 @@ inline int tersoff_zclass(int z) { return z <= 4 ? 4 : (z <= 8 ? 8 : (z <= 16 ? 
 
 // The pair expansion of a rigid-ion or NN2B training set (spectral.cu): the distance range of each
 // pair type in pieces, on each of which the pair energy is a Chebyshev series.
-constexpr int kSpecMaxPieces = 32;
+constexpr int kSpecMaxPieces = 16;
 constexpr int kSpecMaxK = 96;         // terms of a piece (a multiple of 8)
 constexpr int kSpecMaxCols = 1024;    // columns of all pieces and of the linear terms
-constexpr int kSpecEvBlocks = 12;     // energy/virial configurations per work item
-constexpr int kSpecWarps = 4;
+constexpr int kSpecEvBlocks = 16;     // energy/virial configurations per work item
 struct SpecPiece {
   double mid, half;  // x = (d - mid) / half
   double to;         // the piece holds the pairs of its type with d < to (and not in an earlier piece)
@@ -61,17 +60,19 @@ struct SpecView {
   int ncb, n_lin;           // column blocks of 8: the n_lin linear columns first, then the pieces' terms by degree
   int n_items;              // work items per group of individuals
   int n_part;               // rows of `part`
-  const double* ctab;
-  const double* M;          // [row block][column block][8 x 8]
-  const int* row_block;     // [Nc_force + 1] first row block of each force configuration; then the energy/virial blocks
+  const double* ctab;       // [n_ctab]
+  int n_ctab;
+  const double* M;          // per set of rows (force configuration, then energy/virial item) at moff[set]:
+  const long long* moff;    //   [column block][mnb[set] row blocks][8 x 8]
+  const int* mnb;
   // per plan
-  double* coef;             // [individuals / 8][column block][8 x 8]
-  uint8_t* need;            // [piece][Pstride] column blocks in use
+  double* coef;             // [individuals / 32][column block][4][8 x 8]
+  unsigned long long* need; // [P] column blocks in use of every piece, 4 bits each
   double* part;             // [n_part][Pstride]: squared errors per force configuration, then of the energies
                             // and of the virials per energy/virial item
   int* flagged;             // [P] 1: left to the direct items
-  int* list;                // flagged individuals, *count of them
-  int* count;
+  int* list;                // flagged individuals, count[0] of them (empty between generations)
+  int* count;               // [1]: individuals whose fitness their items have folded
 };
 
 struct DevSet {

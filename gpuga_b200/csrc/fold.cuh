@@ -94,7 +94,11 @@ __device__ __forceinline__ void finish_individuals(const JobView& J, int p, int 
     if (q < 0) continue;  // warp-uniform
     __threadfence();
     fold_fitness(J, q, lane);
-    if (lane == 0) J.fit_count[q] = 0;
+    if (lane == 0) {
+      J.fit_count[q] = 0;
+      // the job's last individual: an empty list of direct individuals for the next generation
+      if (J.sp.count && atomicAdd(J.sp.count + 1, 1) == J.P - 1) J.sp.count[0] = J.sp.count[1] = 0;
+    }
   }
 }
 
