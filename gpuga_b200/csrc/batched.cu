@@ -56,13 +56,6 @@ __global__ void decode_jobs(const JobView* __restrict__ jobs, const int2* __rest
   if (!jobs[jp.x].sp.M) decode_individual(jobs[jp.x], jp.y);
 }
 
-struct Consts {
-  const float* base;
-  int stride;
-  int p;
-  __device__ __forceinline__ float operator[](int k) const { return __ldg(base + (size_t)k * stride + p); }
-};
-
 // --------------------------------------------------------------------------- Tersoff
 // The lane's Tersoff constants.  The pair terms fr = cr e^{-lr t}, fa = ca e^{-la t} come in two
 // forms (tersoff_atom, PM): FP64 with FP64 constants (the FP32 value plus its FP64 remainder), or
@@ -1430,6 +1423,7 @@ JobView make_job_view(const Engine* e, const Plan* plan) {
   j.comps = plan->d_comps;
   j.fit_count = plan->d_fitcnt;
   j.sp = plan->sp;
+  j.ev = plan->ev;
   return j;
 }
 
@@ -1439,9 +1433,12 @@ LaunchSet::~LaunchSet() {
   if (d_items) cudaFree(d_items);
   if (d_indmap) cudaFree(d_indmap);
   if (d_specmap) cudaFree(d_specmap);
-  if (side) cudaStreamDestroy(side);
+  if (d_evgroups) cudaFree(d_evgroups);
+  for (auto x : side)
+    if (x) cudaStreamDestroy(x);
   if (fork) cudaEventDestroy(fork);
-  if (join) cudaEventDestroy(join);
+  for (auto x : join)
+    if (x) cudaEventDestroy(x);
   for (auto ev : tev)
     if (ev) cudaEventDestroy(ev);
 }
@@ -1564,6 +1561,7 @@ int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<I
                   e->h_zmax[c]);
         return GPUGA_ERR_UNSUPPORTED;
       }
+      if (!force && d.ev.pairs) continue;  // pair by pair, below
       // slot-major staged geometry: zc slots per atom of (float4, the FP64 length (FP64 pair terms)
       // or its FP32 remainder, pair set[, reverse position]) + counts
       const bool d64 = (force ? kPairModeForce : kPairModeEV) == kPair64;
@@ -1651,6 +1649,19 @@ int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<I
           {WorkItem{c, p0, pack_G(G, staged, fbytes, global, Grule, force, once), job, gofs}, cf * cnt, (double)Na * cnt, cf * cnt, cs * cnt});
     }
   }
+  if (d.ev.pairs && !only) {
+    const LaunchKey key{0, 0, nmax, 0, lo ? 1 : 0, 1};
+    smem_need[key] = std::max(smem_need[key], tersoff_ev_smem(d.ev));
+    for (const EvItem& x : e->h_ev_items)
+      for (int p0 = 0; p0 < P; p0 += 32) {
+        const double cnt = std::min(32, P - p0);
+        // per pair: twice s 4, b and b' 20 and 24 for the virial; pair terms 30 (44 with two exponentials), 12 more
+        // for the virial
+        const double fl = (lo ? 152.0 : 138.0) * x.pairs * cnt;
+        groups[key].push_back({WorkItem{x.seg, p0, pack_G(32, false, 0, false, 32, false), job, x.n_segs}, fl,
+                               (double)x.atoms * cnt, fl, 0.0});
+      }
+  }
   if (d.sp.M) {
     // the pair expansion's items: a force configuration, or up to kSpecEvBlocks energy/virial ones, x 32
     // individuals; the direct items above then take only the individuals that it leaves to them
@@ -1686,6 +1697,8 @@ int launch_one(const LaunchSet* ls, const Launch& L, cudaStream_t st, bool confi
   const dim3 grid(L.count), block(kBlock);
   const dim3 pgrid(L.fallback ? std::min(L.count, kFallbackGrid) : L.count);
   const WorkItem* items = ls->d_items + L.first;
+  if (L.expansion && L.kind == 0)
+    return tersoff_ev_items_launch(ls->d_jobs, items, L.count, L.smem, L.nmax, L.lo, configure_only, st);
   if (L.expansion) return configure_only ? GPUGA_OK : spectral_items_launch(ls->d_jobs, items, L.count, st);
 #define GPUGA_TERSOFF1(ZC, NT)                                                          \
   do {                                                                                  \
@@ -1741,7 +1754,7 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
                     const std::vector<std::pair<const float*, double*>>* targets, const std::vector<char>* only) {
   std::map<LaunchKey, std::vector<ItemSpec>> groups;
   std::map<LaunchKey, size_t> smem_need;
-  std::vector<int2> indmap, specmap, by_class[5];
+  std::vector<int2> indmap, specmap, by_class[5], evgroups;
   ls->jobs.clear();
   bool plain_pairs[3] = {false, false, false};  // some job of the kind evaluates every pair directly
   for (size_t j = 0; j < jobs.size(); ++j) {
@@ -1778,11 +1791,15 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
       plan->gscratch_floats = need;
     }
     ls->jobs.push_back(make_job_view(e, plan));
+    if (only) ls->jobs.back().ev = TersoffEvView{};  // a partial set has no tables
     if (targets) {  // the job's population / fitness live elsewhere (a device GA's buffers)
       ls->jobs.back().pop = (*targets)[j].first;
       ls->jobs.back().fitness = (*targets)[j].second;
     }
     for (int p = 0; p < jobs[j].second->P; ++p) indmap.push_back(make_int2((int)j, p));
+    if (plan->ev.pairs && !only) {
+      for (int g = 0; g < (plan->P + 31) / 32; ++g) evgroups.push_back(make_int2((int)j, g));
+    }
     if (plan->sp.M) {
       for (int p = 0; p < plan->P; ++p) by_class[spectral_class(e->d)].push_back(make_int2((int)j, p));
     } else if (e->d.potential_type != 1 && e->d.potential_type != 2) {
@@ -1837,6 +1854,11 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
     ls->spec_class[k] = (int)by_class[k].size();
     specmap.insert(specmap.end(), by_class[k].begin(), by_class[k].end());
   }
+  ls->ev_groups = (int)evgroups.size();
+  if (!evgroups.empty()) {
+    GPUGA_CUDA(cudaMalloc(&ls->d_evgroups, sizeof(int2) * evgroups.size()));
+    GPUGA_CUDA(cudaMemcpy(ls->d_evgroups, evgroups.data(), sizeof(int2) * evgroups.size(), cudaMemcpyHostToDevice));
+  }
   ls->spec_individuals = (int)specmap.size();
   if (!specmap.empty()) {
     GPUGA_CUDA(cudaMalloc(&ls->d_specmap, sizeof(int2) * specmap.size()));
@@ -1845,9 +1867,9 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
   GPUGA_CUDA(cudaMalloc(&ls->d_jobs, sizeof(JobView) * std::max<size_t>(ls->jobs.size(), 1)));
   GPUGA_CUDA(cudaMallocHost(&ls->h_jobs, sizeof(JobView) * std::max<size_t>(ls->jobs.size(), 1)));
   GPUGA_CUDA(cudaMemcpy(ls->d_jobs, ls->jobs.data(), sizeof(JobView) * ls->jobs.size(), cudaMemcpyHostToDevice));
-  GPUGA_CUDA(cudaStreamCreateWithFlags(&ls->side, cudaStreamNonBlocking));
+  for (auto& x : ls->side) GPUGA_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
   GPUGA_CUDA(cudaEventCreateWithFlags(&ls->fork, cudaEventDisableTiming));
-  GPUGA_CUDA(cudaEventCreateWithFlags(&ls->join, cudaEventDisableTiming));
+  for (auto& x : ls->join) GPUGA_CUDA(cudaEventCreateWithFlags(&x, cudaEventDisableTiming));
   ls->tev.assign(2 * ls->launches.size(), nullptr);
   for (auto& ev : ls->tev) GPUGA_CUDA(cudaEventCreate(&ev));
   ls->t_ms.assign(ls->launches.size(), 0.0);
@@ -1883,35 +1905,53 @@ int launchset_collect_timing(LaunchSet* ls) {
   return GPUGA_OK;
 }
 
-// One generation of every job of the set: decode, the batched launches
-// (energy/virial launches on `st`, force launches on the side stream), then
-// the fitness fold.  While per-launch timing is on, every launch runs on `st`
-// one after another, so that each event pair brackets that launch alone.
+// One generation of every job of the set: decode, tables and coefficients, the batched launches, then
+// the fitness fold.  The launches of a set run side by side, the longest on `st`, the others in turn on the side
+// streams (pair-by-pair Tersoff items on the first, behind their tables, which run beside the decode): a launch's
+// last CTAs then share the GPU with the next one.  While per-launch timing is on, every launch runs on `st` one
+// after another, so that each event pair brackets that launch alone.
 int launchset_enqueue(LaunchSet* ls, cudaStream_t st) {
   const int total = ls->total_individuals;
+  int used = 0;  // side streams in use
+  auto fork_to = [&](int n) -> int {
+    GPUGA_CUDA(cudaEventRecord(ls->fork, st));
+    for (int k = 0; k < n; ++k) GPUGA_CUDA(cudaStreamWaitEvent(ls->side[k], ls->fork, 0));
+    used = std::max(used, n);
+    return GPUGA_OK;
+  };
+  const bool ev_side = ls->ev_groups > 0 && !ls->timing;
+  if (ev_side) GPUGA_TRY(fork_to(1));
+  if (ls->ev_groups > 0) GPUGA_TRY(tersoff_tables_launch(ls, ev_side ? ls->side[0] : st));
   if (total > ls->spec_individuals) {
     decode_jobs<<<(total + 127) / 128, 128, 0, st>>>(ls->d_jobs, ls->d_indmap, total);
     GPUGA_CUDA(cudaGetLastError());
   }
   if (ls->spec_individuals > 0) GPUGA_TRY(spectral_coefficients(ls, st));
-  // several launches (job mixes with several kernel classes): every second one on the side stream
-  const bool any_side = ls->launches.size() > 1 && !ls->timing;
-  if (any_side) {
-    GPUGA_CUDA(cudaEventRecord(ls->fork, st));
-    GPUGA_CUDA(cudaStreamWaitEvent(ls->side, ls->fork, 0));
-  }
+  const int n_launch = (int)ls->launches.size();
+  if (n_launch > 1 && !ls->timing) GPUGA_TRY(fork_to(std::min(n_launch - 1, kSideStreams)));
+  else if (ev_side) GPUGA_TRY(fork_to(1));
   GPUGA_TRY(launchset_collect_timing(ls));
-  for (size_t k = 0; k < ls->launches.size(); ++k) {
+  int turn = 0;  // 0: st, then the side streams
+  for (int k = 0; k < n_launch; ++k) {
     const Launch& L = ls->launches[k];
-    cudaStream_t s = any_side && ((k & 1) || L.fallback) ? ls->side : st;
+    cudaStream_t s = st;
+    if (!ls->timing) {
+      if (L.expansion && L.kind == 0) {
+        s = ls->side[0];
+      } else {
+        if (ev_side && turn == 1 && n_launch > 2) ++turn;  // the first side stream is taken
+        s = turn == 0 || used < turn ? st : ls->side[turn - 1];
+        turn = turn >= used ? 0 : turn + 1;
+      }
+    }
     if (ls->timing) GPUGA_CUDA(cudaEventRecord(ls->tev[2 * k], s));
     GPUGA_TRY(launch_one(ls, L, s, false));
     if (ls->timing) GPUGA_CUDA(cudaEventRecord(ls->tev[2 * k + 1], s));
   }
   ls->t_pending = ls->timing;
-  if (any_side) {
-    GPUGA_CUDA(cudaEventRecord(ls->join, ls->side));
-    GPUGA_CUDA(cudaStreamWaitEvent(st, ls->join, 0));
+  for (int k = 0; k < used; ++k) {
+    GPUGA_CUDA(cudaEventRecord(ls->join[k], ls->side[k]));
+    GPUGA_CUDA(cudaStreamWaitEvent(st, ls->join[k], 0));
   }
   if (!ls->folds) {  // a partial set: the fitness of every individual in one more launch
     fitness_jobs<<<(total + 3) / 4, 128, 0, st>>>(ls->d_jobs, ls->d_indmap, total);
@@ -2010,6 +2050,7 @@ int plan_build(Engine* e, int P, Plan** out) {
   GPUGA_TRY(e->alloc(&plan->d_comps, (size_t)3 * P));
   GPUGA_TRY(e->alloc(&plan->d_fitcnt, (size_t)P));
   if (d.sp.M) GPUGA_TRY(spectral_plan(e, plan.get()));
+  if (d.ev.pairs) GPUGA_TRY(tersoff_ev_plan(e, plan.get()));
   GPUGA_CUDA(cudaMemset(plan->d_fitcnt, 0, sizeof(int) * (size_t)P));
   GPUGA_TRY(e->alloc(&plan->d_pop, (size_t)P * d.num_vars));
   GPUGA_CUDA(cudaMallocHost(&plan->h_pop, sizeof(float) * (size_t)P * d.num_vars));

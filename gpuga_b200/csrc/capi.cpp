@@ -286,7 +286,8 @@ int gpuga_plan_kernels(gpuga_engine* h, int P, int* kernels) {
   if (s != GPUGA_OK) return s;
   const LaunchSet* ls = plan->ls.get();
   // decode and pair coefficients, items (+ fitness fold)
-  *kernels = (ls->total_individuals > ls->spec_individuals) + (int)ls->launches.size() + (ls->folds ? 0 : 1);
+  *kernels = (ls->total_individuals > ls->spec_individuals) + (ls->ev_groups > 0) +
+             (int)ls->launches.size() + (ls->folds ? 0 : 1);
   for (int n : ls->spec_class) *kernels += n > 0;
   return GPUGA_OK;
 }

@@ -105,4 +105,11 @@ __device__ __forceinline__ void decode_individual(const JobView& J, int p) {
   }
 }
 
+struct Consts {
+  const float* base;
+  int stride;
+  int p;
+  __device__ __forceinline__ float operator[](int k) const { return __ldg(base + (size_t)k * stride + p); }
+};
+
 }  // namespace gpuga

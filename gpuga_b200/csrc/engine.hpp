@@ -75,7 +75,42 @@ struct SpecView {
   int* count;               // [1]: individuals whose fitness their items have folded
 };
 
+// Pair-by-pair energy/virial items of the minimal Tersoff potential (tersoff_ev.cu).
+constexpr int kEvSegPairs = 240;  // pairs of a segment, and of an item, at most (12 warps x 10 batches x 2)
+struct TersoffSegment {
+  int config, b0, n;
+  int part;  // row of TersoffEvView::part, or -1: the configuration's only segment writes its results
+};
+struct alignas(16) EvPair {  // coefficients of an unordered pair and its two bonds (tersoff_ev.cu)
+  double A[2], B[2], C[2];   // s(dh) = A + dh (B + dh C)
+  double delta;              // d less its grid point
+  double hfc, hfcp;          // fc / 2, fc' / 2
+  float hfc32;
+  int code;                  // grid point, pair set, shell
+  float D[6];                // d u (x) u: xx yy zz xy yz zx
+  float X[2][2][6];          // [bond][power of dh]: ds / d(strain) = X0 + dh (X1 + dh X2)
+  float pad[2];
+};
+static_assert(sizeof(EvPair) == 208, "13 x 16 bytes");
+struct TersoffEvView {
+  const EvPair* pairs;
+  const float4* shell;   // [pair][bond][2]: X2
+  const TersoffSegment* segs;
+  const int* seg0;       // [Nc + 1] first row of `part` of each configuration
+  float h0;
+  int tab_base, tab_n;   // b(s): first entry (top 12 bits of the FP32 s) and entries
+  int exp_base, exp_n, n_exp;  // exponentials: first grid point, grid points, tables
+  int n_part, n_items;   // items per group of 32 individuals
+  // per plan
+  unsigned char* tables; // [individuals / 32]
+  double* part;          // [n_part][7][Pstride]
+};
+struct EvItem {
+  int seg, n_segs, pairs, atoms;
+};
+
 struct DevSet {
+  TersoffEvView ev{};          // ev.pairs == nullptr: energy/virial items atom by atom (batched.cu)
   SpecView sp{};               // sp.M == nullptr: every pair is evaluated directly
   int Nc = 0, Nc_force = 0, N = 0, N_force = 0, B = 0, max_Na = 0, max_Z = 0;
   int potential_type = -1, num_types = 1, num_neurons = 0, num_vars = 0;
@@ -200,6 +235,7 @@ struct JobView {
                          // item that finishes an individual's last one folds its fitness (reset to
                          // 0 there).  Null: a partial launch set (no fold).
   SpecView sp;           // sp.M == nullptr: no pair expansion
+  TersoffEvView ev;      // ev.pairs == nullptr: no pair-by-pair items
 };
 
 struct Launch {
@@ -218,6 +254,8 @@ struct Launch {
   double sfu = 0;      // transcendental calls per launch
 };
 
+constexpr int kSideStreams = 3;
+
 // Launches of one generation over one or more jobs (a job table on the device).
 struct LaunchSet {
   std::vector<Launch> launches;
@@ -230,9 +268,11 @@ struct LaunchSet {
   int2* d_specmap = nullptr;   // the individuals of jobs with a pair expansion -> (job, p), by kernel class
   int spec_class[5] = {0, 0, 0, 0, 0};  // how many of each (spectral_class)
   int spec_individuals = 0;
+  int2* d_evgroups = nullptr;  // groups of 32 individuals of jobs with pair-by-pair Tersoff items -> (job, group)
+  int ev_groups = 0;
   bool folds = true;           // the items fold every individual's fitness (no fitness_jobs launch)
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
+  cudaStream_t side[kSideStreams] = {};  // launches of one generation side by side
+  cudaEvent_t fork = nullptr, join[kSideStreams] = {};
   bool timing = false;               // event pair around every launch (eager launches)
   std::vector<cudaEvent_t> tev;      // 2 per launch
   std::vector<double> t_ms;          // accumulated device time per launch
@@ -266,6 +306,7 @@ struct Plan {
   double* d_res = nullptr;     // [P][Nc][kResK]
   double* d_fitness = nullptr; // [P]
   double* d_comps = nullptr;   // [P][3]
+  TersoffEvView ev{};          // pair-by-pair items: the training set's view with this plan's buffers
   SpecView sp{};               // pair expansion: the training set's view with this plan's buffers
   int* d_fitcnt = nullptr;     // [P] per-generation completion counts (JobView::fit_count)
   float* d_pop = nullptr;      // [P][d] staging
@@ -293,6 +334,7 @@ struct Engine {
   float* d_pmin = nullptr;
   float* d_pmax = nullptr;
   std::vector<int> h_NN, h_off, h_nbr, h_zmax;  // host copies of the neighbor list
+  std::vector<EvItem> h_ev_items;               // pair-by-pair Tersoff items of a group of individuals
   std::vector<int> h_spec_blocks;               // pair expansion: 8 x 8 products per force configuration
   std::vector<char> h_pair_sym;                 // NN2B: per configuration, bond list symmetric
   std::map<int, std::unique_ptr<Plan>> plans;    // keyed by population size
@@ -330,6 +372,15 @@ int spectral_class(const DevSet& d);           // 0 rigid ion, 1-4 network width
 int spectral_coefficients(const LaunchSet* ls, cudaStream_t st);
 int spectral_items_launch(const JobView* jobs, const WorkItem* items, int count, cudaStream_t st);
 
+// tersoff_ev.cu
+int tersoff_ev_build(Engine* e);
+int tersoff_ev_plan(Engine* e, Plan* plan);
+size_t tersoff_ev_smem(const TersoffEvView& v);
+size_t tersoff_ev_table_bytes(const TersoffEvView& v);
+int tersoff_tables_launch(const LaunchSet* ls, cudaStream_t st);  // tables and decode
+int tersoff_ev_items_launch(const JobView* jobs, const WorkItem* items, int count, size_t smem, int num_types, bool lo,
+                            bool configure, cudaStream_t st);
+
 // geometry.cu
 int build_geometry(Engine* e);
 // FP32 neighbor rule of neighbor.cu:30-66 on reference-layout device arrays.
@@ -363,7 +414,7 @@ JobView make_job_view(const Engine* e, const Plan* plan);
 int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSet* ls,
                     const std::vector<std::pair<const float*, double*>>* targets = nullptr,
                     const std::vector<char>* only = nullptr);
-// Enqueues one generation of every job of the set on `st` (force launches on a side stream).
+// Enqueues one generation of every job of the set on `st` and the set's side streams.
 int launchset_enqueue(LaunchSet* ls, cudaStream_t st);
 int launchset_collect_timing(LaunchSet* ls);
 // Points job row `job` at new population / fitness / force-dump buffers (enqueued on `st`).

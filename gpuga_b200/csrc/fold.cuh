@@ -30,7 +30,25 @@ __device__ __forceinline__ void fold_fitness(const JobView& J, int p, int lane) 
   }
   for (int c = expanded ? Nc : lane; c < Nc; c += 32) {
     const double* r = res + ((size_t)p * Nc + c) * kResK;
-    if (c >= Nc_force) {
+    if (c >= Nc_force && J.ev.pairs && J.ev.seg0[c + 1] > J.ev.seg0[c]) {
+      // a configuration in several segments: their sums in order are its results
+      double v[7];
+#pragma unroll
+      for (int k = 0; k < 7; ++k) v[k] = 0.0;
+      for (int s = J.ev.seg0[c]; s < J.ev.seg0[c + 1]; ++s)
+#pragma unroll
+        for (int k = 0; k < 7; ++k) v[k] += __ldcg(J.ev.part + ((size_t)s * 7 + k) * J.Pstride + p);
+      double* w = J.res + ((size_t)p * Nc + c) * kResK;
+#pragma unroll
+      for (int k = 0; k < 7; ++k) w[k] = v[k];
+      const double de = v[0] - E_ref[c];
+      eE = __fma_rn(de, de, eE);
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const double dw = v[1 + k] - W_ref[c + (size_t)Nc * k];
+        eW = __fma_rn(dw, dw, eW);
+      }
+    } else if (c >= Nc_force) {
       const double de = __ldcg(r) - E_ref[c];
       eE = __fma_rn(de, de, eE);
 #pragma unroll
@@ -82,7 +100,8 @@ __device__ __forceinline__ void finish_individuals(const JobView& J, int p, int 
     if (threadIdx.x < G && p >= 0) {
       // items that count for p: one per configuration, or the expansion's items and, for an
       // individual that it handed to the direct items, theirs as well
-      const int total = J.sp.part ? J.sp.n_items + (__ldcg(J.sp.flagged + p) ? J.v.Nc : 0) : J.v.Nc;
+      const int total = J.sp.part ? J.sp.n_items + (__ldcg(J.sp.flagged + p) ? J.v.Nc : 0)
+                                  : (J.ev.pairs ? J.Nc_force + J.ev.n_items : J.v.Nc);
       if (atomic_add_acq_rel(&J.fit_count[p], 1) == total - 1) last = p;
     }
     s_last[threadIdx.x] = last;
