@@ -1424,6 +1424,7 @@ JobView make_job_view(const Engine* e, const Plan* plan) {
   j.fit_count = plan->d_fitcnt;
   j.sp = plan->sp;
   j.ev = plan->ev;
+  j.tf = d.tf;
   return j;
 }
 
@@ -1454,7 +1455,7 @@ struct ItemSpec {
   double cost, units, flops, sfu;
 };
 struct LaunchKey {
-  int kind, zclass, nmax, force, lo, expansion;
+  int kind, zclass, nmax, force, lo, expansion;  // expansion: 1 pair expansion or Tersoff pairs, 2 packed Tersoff forces
   bool operator<(const LaunchKey& o) const {
     return std::tie(kind, zclass, nmax, force, lo, expansion) <
            std::tie(o.kind, o.zclass, o.nmax, o.force, o.lo, o.expansion);
@@ -1562,6 +1563,22 @@ int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<I
         return GPUGA_ERR_UNSUPPORTED;
       }
       if (!force && d.ev.pairs) continue;  // pair by pair, below
+      if (force && e->h_tf[c]) {  // packed items (tersoff_force.cu); their one tile is the rule's for every tile option
+        const LaunchKey key{0, 0, nmax, 0, lo ? 1 : 0, 2};
+        smem_need[key] = std::max(smem_need[key], tersoff_force_smem(Na));
+        double cf = 0, cs = 0;
+        for (int k = 0; k < Na; ++k) {
+          cf += atom_flops[ts.Na_sum[c] + k];
+          cs += atom_sfu[ts.Na_sum[c] + k];
+        }
+        const int G = 2 << tersoff_force_lgH(Na);
+        for (int p0 = 0; p0 < P; p0 += G) {
+          const int cnt = std::min(G, P - p0);
+          groups[key].push_back(
+              {WorkItem{c, p0, pack_G(G, false, 0, false, G, true), job, 0}, cf * cnt, (double)Na * cnt, cf * cnt, cs * cnt});
+        }
+        continue;
+      }
       // slot-major staged geometry: zc slots per atom of (float4, the FP64 length (FP64 pair terms)
       // or its FP32 remainder, pair set[, reverse position]) + counts
       const bool d64 = (force ? kPairModeForce : kPairModeEV) == kPair64;
@@ -1697,6 +1714,7 @@ int launch_one(const LaunchSet* ls, const Launch& L, cudaStream_t st, bool confi
   const dim3 grid(L.count), block(kBlock);
   const dim3 pgrid(L.fallback ? std::min(L.count, kFallbackGrid) : L.count);
   const WorkItem* items = ls->d_items + L.first;
+  if (L.packed) return tersoff_force_launch(ls->d_jobs, items, L.count, L.smem, L.nmax, L.lo, configure_only, st);
   if (L.expansion && L.kind == 0)
     return tersoff_ev_items_launch(ls->d_jobs, items, L.count, L.smem, L.nmax, L.lo, configure_only, st);
   if (L.expansion) return configure_only ? GPUGA_OK : spectral_items_launch(ls->d_jobs, items, L.count, st);
@@ -1816,7 +1834,8 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
     L.zclass = kv.first.zclass;
     L.nmax = kv.first.nmax;
     L.lo = kv.first.lo != 0;
-    L.expansion = kv.first.expansion != 0;
+    L.expansion = kv.first.expansion == 1;
+    L.packed = kv.first.expansion == 2;
     L.fallback = L.kind != 0 && !L.expansion && !plain_pairs[L.kind];
     int nforce = 0;
     for (auto& t : v) nforce += item_force(t.w) ? 1 : 0;
@@ -2009,7 +2028,8 @@ int tune_tiles(Engine* e, Plan* plan) {
   fill_value<<<(unsigned)((npop + 255) / 256), 256, 0, st>>>(plan->d_pop, npop, 0.5f);  // mid-range individuals
   GPUGA_CUDA(cudaGetLastError());
   std::map<int, std::vector<int>> classes;
-  for (int c = 0; c < ts.Nc_force; ++c) classes[ts.Na[c]].push_back(c);
+  for (int c = 0; c < ts.Nc_force; ++c)
+    if (!e->h_tf[c]) classes[ts.Na[c]].push_back(c);  // the packed items have one tile
   plan->tiles.assign(ts.Nc, 0);
   for (int c = 0; c < ts.Nc_force; ++c) plan->tiles[c] = kTileDefault;
   for (const auto& kv : classes) {
@@ -2046,6 +2066,8 @@ int plan_build(Engine* e, int P, Plan** out) {
   if (const int K64 = consts64_per_individual(d)) GPUGA_TRY(e->alloc(&plan->d_consts64, (size_t)K64 * plan->Pstride));
   if (d.potential_type == 3) GPUGA_TRY(e->alloc(&plan->d_weights, (size_t)d.num_vars * plan->Pstride));
   GPUGA_TRY(e->alloc(&plan->d_res, (size_t)P * d.Nc * kResK));
+  // (items write the components they own; the others stay zero)
+  GPUGA_CUDA(cudaMemset(plan->d_res, 0, sizeof(double) * (size_t)P * d.Nc * kResK));
   GPUGA_TRY(e->alloc(&plan->d_fitness, (size_t)P));
   GPUGA_TRY(e->alloc(&plan->d_comps, (size_t)3 * P));
   GPUGA_TRY(e->alloc(&plan->d_fitcnt, (size_t)P));

@@ -105,11 +105,24 @@ struct TersoffEvView {
   unsigned char* tables; // [individuals / 32]
   double* part;          // [n_part][7][Pstride]
 };
+// Packed force items of the minimal Tersoff potential (tersoff_force.cu): per configuration its atoms in the order of
+// `atom` (four bonds inside R1 first), slot j of the k-th at base + j Na + k.
+struct TersoffForceView {
+  const float4* gu;  // unit vector, d
+  const float4* gd;  // 1 / d (negative: pair set 1), d - (float)d, fc, fc'
+  const int* rev;    // slot * Na + place of the reverse bond
+  const double* ref; // [atom][3] reference force
+  const int* base;
+  const int* inner;  // atoms with four bonds inside R1
+  const int* lgH;    // log2 of the pairs of individuals per item
+  const int* atom;   // atom of each place
+};
 struct EvItem {
   int seg, n_segs, pairs, atoms;
 };
 
 struct DevSet {
+  TersoffForceView tf{};       // packed force items (Engine::h_tf: which configurations)
   TersoffEvView ev{};          // ev.pairs == nullptr: energy/virial items atom by atom (batched.cu)
   SpecView sp{};               // sp.M == nullptr: every pair is evaluated directly
   int Nc = 0, Nc_force = 0, N = 0, N_force = 0, B = 0, max_Na = 0, max_Z = 0;
@@ -235,12 +248,14 @@ struct JobView {
                          // item that finishes an individual's last one folds its fitness (reset to
                          // 0 there).  Null: a partial launch set (no fold).
   SpecView sp;           // sp.M == nullptr: no pair expansion
+  TersoffForceView tf;
   TersoffEvView ev;      // ev.pairs == nullptr: no pair-by-pair items
 };
 
 struct Launch {
   int kind = 0;        // 0 Tersoff, 1 RI, 2 NN2B
-  bool expansion = false;  // RI / NN2B items of the pair expansion (spectral.cu)
+  bool expansion = false;  // items of the pair expansion (spectral.cu), Tersoff: of pairs (tersoff_ev.cu)
+  bool packed = false;     // packed Tersoff force items (tersoff_force.cu)
   bool fallback = false;   // RI / NN2B direct items that only take the individuals the expansion left
   int zclass = 4;      // Tersoff register-array size
   int nmax = 0;        // NN2B register-array size; Tersoff: number of atom types
@@ -334,6 +349,7 @@ struct Engine {
   float* d_pmin = nullptr;
   float* d_pmax = nullptr;
   std::vector<int> h_NN, h_off, h_nbr, h_zmax;  // host copies of the neighbor list
+  std::vector<char> h_tf;                       // per configuration: its force items are packed ones
   std::vector<EvItem> h_ev_items;               // pair-by-pair Tersoff items of a group of individuals
   std::vector<int> h_spec_blocks;               // pair expansion: 8 x 8 products per force configuration
   std::vector<char> h_pair_sym;                 // NN2B: per configuration, bond list symmetric
@@ -380,6 +396,13 @@ size_t tersoff_ev_table_bytes(const TersoffEvView& v);
 int tersoff_tables_launch(const LaunchSet* ls, cudaStream_t st);  // tables and decode
 int tersoff_ev_items_launch(const JobView* jobs, const WorkItem* items, int count, size_t smem, int num_types, bool lo,
                             bool configure, cudaStream_t st);
+
+// tersoff_force.cu
+int tersoff_force_build(Engine* e);
+int tersoff_force_lgH(int Na);
+size_t tersoff_force_smem(int Na);
+int tersoff_force_launch(const JobView* jobs, const WorkItem* items, int count, size_t smem, int num_types, bool lo,
+                         bool configure, cudaStream_t st);
 
 // geometry.cu
 int build_geometry(Engine* e);

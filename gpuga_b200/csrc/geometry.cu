@@ -782,6 +782,7 @@ int build_geometry(Engine* e) {
     if (!hb.empty()) GPUGA_CUDA(cudaMemcpy(d.hb, hb.data(), sizeof(int) * hb.size(), cudaMemcpyHostToDevice));
     GPUGA_CUDA(cudaMemcpy(d.hb_off, hb_off.data(), sizeof(int) * (Nc + 1), cudaMemcpyHostToDevice));
   }
+  GPUGA_TRY(tersoff_force_build(e));
   GPUGA_TRY(tersoff_ev_build(e));
   return spectral_build(e);
 }
