@@ -1314,16 +1314,32 @@ __global__ void __launch_bounds__(kBlock, KIND == 1 ? 3 : 2) pair_batched(const 
 }
 
 // --------------------------------------------------------------------------- fitness
-// The fitness of every individual in a launch of its own: for launch sets that compute only part
-// of the configurations' results (full sets fold in their work items, finish_item).
-__global__ void fitness_jobs(const JobView* __restrict__ jobs, const int2* __restrict__ indmap, int total) {
-  const int t = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-  if (t >= total) return;
-  const int2 jp = indmap[t];
-  const JobView& J = jobs[jp.x];
-  // every direct item of this generation is done: an empty list for the next one
-  if (jp.y == 0 && J.sp.count && (threadIdx.x & 31) == 0) *J.sp.count = 0;
-  fold_fitness(J, jp.y, threadIdx.x & 31);
+// The fitness of every individual in a launch of its own (fold.cuh).  What bounds it: L2 requests.  The segments' and
+// the expansion's sums lie individual by individual, so a CTA takes 8 individuals and its threads 8 t .. 8 t + 7 lane t
+// of each: a 32-byte sector serves four of them, where a warp per individual fetched it for one.  The sums then
+// go through shared memory to a warp per individual for the butterfly: the order of every sum is that of fold_fitness.
+constexpr int kFoldInd = 8;
+__global__ void __launch_bounds__(32 * kFoldInd) fitness_jobs(const JobView* __restrict__ jobs,
+                                                              const int2* __restrict__ indmap, int total) {
+  __shared__ double s[3][kFoldInd][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int i = threadIdx.x % kFoldInd, c = threadIdx.x / kFoldInd, t = blockIdx.x * kFoldInd + i;
+  if (t < total) {
+    const int2 jp = indmap[t];
+    const JobView& J = jobs[jp.x];
+    // every direct item of this generation is done: an empty list for the next one
+    if (jp.y == 0 && J.sp.count && c == 0) *J.sp.count = 0;
+    double eE, eW, eF;
+    fold_sums(J, jp.y, c, eE, eW, eF);
+    s[0][i][c] = eE;
+    s[1][i][c] = eW;
+    s[2][i][c] = eF;
+  }
+  __syncthreads();
+  const int u = blockIdx.x * kFoldInd + warp;
+  if (u >= total) return;  // warp-uniform
+  const int2 jp = indmap[u];
+  fold_result(jobs[jp.x], jp.y, lane, s[0][warp][lane], s[1][warp][lane], s[2][warp][lane]);
 }
 
 // --------------------------------------------------------------------------- planning
@@ -1973,7 +1989,7 @@ int launchset_enqueue(LaunchSet* ls, cudaStream_t st) {
     GPUGA_CUDA(cudaStreamWaitEvent(st, ls->join[k], 0));
   }
   if (!ls->folds) {  // a partial set: the fitness of every individual in one more launch
-    fitness_jobs<<<(total + 3) / 4, 128, 0, st>>>(ls->d_jobs, ls->d_indmap, total);
+    fitness_jobs<<<(total + kFoldInd - 1) / kFoldInd, 32 * kFoldInd, 0, st>>>(ls->d_jobs, ls->d_indmap, total);
     GPUGA_CUDA(cudaGetLastError());
   }
   return GPUGA_OK;

@@ -5,19 +5,19 @@
 
 namespace gpuga {
 
-// fitness.cu:329-331, 437-555 in FP64 for individual p, by one warp: lane c sums configurations
-// c, c + 32, ... in order, then a butterfly; the same order whichever warp or launch folds, and
-// the same operations: every product and sum is an explicit intrinsic, so that the compiler's
+// fitness.cu:329-331, 437-555 in FP64 for individual p, by 32 lanes: lane c sums configurations
+// c, c + 32, ... in order (fold_sums), then a butterfly (fold_result, a warp); the same order whichever warp or
+// launch folds, and the same operations: every product and sum is an explicit intrinsic, so that the compiler's
 // choice of contracting a * b + c into an FMA cannot differ between the kernels this is inlined in.
 // Reads go through L2 (ld.cg): other CTAs of the same launch wrote the results.
-__device__ __forceinline__ void fold_fitness(const JobView& J, int p, int lane) {
+__device__ __forceinline__ void fold_sums(const JobView& J, int p, int lane, double& eE, double& eW, double& eF) {
   const int Nc = J.v.Nc, Nc_force = J.Nc_force;
   const double* res = J.res;
   // force errors of an individual that the pair expansion evaluated (spectral.cu)
   const bool expanded = J.sp.part && !__ldcg(J.sp.flagged + p);
   const double* __restrict__ E_ref = J.E_ref;
   const double* __restrict__ W_ref = J.W_ref;
-  double eE = 0, eW = 0, eF = 0;
+  eE = eW = eF = 0;
   if (expanded) {
     // the items' sums: force configurations, then the energies and the virials per energy/virial item
     const double* part = J.sp.part + p;
@@ -40,7 +40,8 @@ __device__ __forceinline__ void fold_fitness(const JobView& J, int p, int lane) 
         for (int k = 0; k < 7; ++k) v[k] += __ldcg(J.ev.part + ((size_t)s * 7 + k) * J.Pstride + p);
       double* w = J.res + ((size_t)p * Nc + c) * kResK;
 #pragma unroll
-      for (int k = 0; k < 7; ++k) w[k] = v[k];
+      for (int k = 0; k < 6; k += 2) *reinterpret_cast<double2*>(w + k) = double2{v[k], v[k + 1]};
+      w[6] = v[6];
       const double de = v[0] - E_ref[c];
       eE = __fma_rn(de, de, eE);
 #pragma unroll
@@ -60,6 +61,10 @@ __device__ __forceinline__ void fold_fitness(const JobView& J, int p, int lane) 
       eF += __ldcg(r + 7);
     }
   }
+}
+
+// The fitness of individual p from its lanes' sums, by a warp.
+__device__ __forceinline__ void fold_result(const JobView& J, int p, int lane, double eE, double eW, double eF) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     eE += __shfl_xor_sync(0xffffffffu, eE, o);
@@ -76,6 +81,12 @@ __device__ __forceinline__ void fold_fitness(const JobView& J, int p, int lane) 
       J.comps[3 * (size_t)p + 2] = rF;
     }
   }
+}
+
+__device__ __forceinline__ void fold_fitness(const JobView& J, int p, int lane) {
+  double eE, eW, eF;
+  fold_sums(J, p, lane, eE, eW, eF);
+  fold_result(J, p, lane, eE, eW, eF);
 }
 
 // End of every work item: its results for individuals p0 .. p0 + G - 1 are written.  Each of those
