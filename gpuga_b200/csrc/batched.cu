@@ -1,5 +1,8 @@
 // Batched fitness evaluation: every individual x every configuration of the
-// training set per generation.
+// training set per generation.  The items here are the general ones: pair expansions
+// (spectral.cu), Tersoff energies and virials pair by pair (tersoff_ev.cu) and packed
+// Tersoff forces (tersoff_force.cu) take the configurations that their rules name, in
+// the launches that are planned and enqueued here.
 //
 // Decomposition.  A work item is (configuration c, group of G individuals).
 // Inside a CTA each warp lane is one individual (G = 32) or, for force
@@ -1471,7 +1474,7 @@ struct ItemSpec {
   double cost, units, flops, sfu;
 };
 struct LaunchKey {
-  int kind, zclass, nmax, force, lo, expansion;  // expansion: 1 pair expansion or Tersoff pairs, 2 packed Tersoff forces
+  int kind, zclass, nmax, force, lo, expansion;  // expansion: 1 pair expansion or Tersoff pairs, 2, 3 packed Tersoff forces (two sizes of CTA)
   bool operator<(const LaunchKey& o) const {
     return std::tie(kind, zclass, nmax, force, lo, expansion) <
            std::tie(o.kind, o.zclass, o.nmax, o.force, o.lo, o.expansion);
@@ -1580,7 +1583,7 @@ int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<I
       }
       if (!force && d.ev.pairs) continue;  // pair by pair, below
       if (force && e->h_tf[c]) {  // packed items (tersoff_force.cu); their one tile is the rule's for every tile option
-        const LaunchKey key{0, 0, nmax, 0, lo ? 1 : 0, 2};
+        const LaunchKey key{0, 0, nmax, 0, lo ? 1 : 0, tersoff_force_large(Na) ? 3 : 2};
         smem_need[key] = std::max(smem_need[key], tersoff_force_smem(Na));
         double cf = 0, cs = 0;
         for (int k = 0; k < Na; ++k) {
@@ -1851,7 +1854,7 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
     L.nmax = kv.first.nmax;
     L.lo = kv.first.lo != 0;
     L.expansion = kv.first.expansion == 1;
-    L.packed = kv.first.expansion == 2;
+    L.packed = kv.first.expansion >= 2;
     L.fallback = L.kind != 0 && !L.expansion && !plain_pairs[L.kind];
     int nforce = 0;
     for (auto& t : v) nforce += item_force(t.w) ? 1 : 0;

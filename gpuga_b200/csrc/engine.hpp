@@ -400,6 +400,7 @@ int tersoff_ev_items_launch(const JobView* jobs, const WorkItem* items, int coun
 // tersoff_force.cu
 int tersoff_force_build(Engine* e);
 int tersoff_force_lgH(int Na);
+bool tersoff_force_large(int Na);  // in CTAs of the larger size
 size_t tersoff_force_smem(int Na);
 int tersoff_force_launch(const JobView* jobs, const WorkItem* items, int count, size_t smem, int num_types, bool lo,
                          bool configure, cudaStream_t st);

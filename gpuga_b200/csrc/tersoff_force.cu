@@ -13,6 +13,9 @@
 // instructions, 200 of them packed, and 40 SFU).  The scalar form in batched.cu issued about 516 per individual and
 // atom: the packed operations halve the arithmetic, and geometry, addresses and cosines are shared by the two.  Bond
 // orders and exponentials come from the SFU (lg2 / ex2 / rcp.approx.ftz) as there, 1 / d from the training set.
+// It issues on about 40 % of cycles: 16 warps per SM (128 registers, the scratch) wait for the geometry from L2 and at the two
+// barriers.  So CTAs are small: four of 128 threads whose phases overlap, 945 us at 1000 individuals x 250 configurations of
+// 8 to 512 atoms, where two of 256 threads with twice the individuals took 1019 us (the scalar form: 1.58 ms).
 #include <algorithm>
 #include <cmath>
 
@@ -24,7 +27,7 @@ namespace gpuga {
 
 namespace {
 
-constexpr int kFThreads = 256, kFWarps = kFThreads / 32;
+constexpr int kFThreads = 128, kFThreadsLarge = 256;  // per CTA: scratch of up to kForceSmem, above
 
 // ------------------------------------------------------------------------------ packed FP32
 typedef unsigned long long f2;
@@ -290,23 +293,23 @@ __device__ __forceinline__ void atom_forces(const ForceConsts<NT, LO>& K, const 
 }
 
 // One CTA: one configuration x G = 2 H individuals, lane = pair of individuals x atom.  First every atom's f_ij into
-// shared memory, then F_i and its squared error in FP64: per thread its atoms in step order, then the 8 warps in order,
+// shared memory, then F_i and its squared error in FP64: per thread its atoms in step order, then the warps in order,
 // then a butterfly over the atom slots of an individual (H is a property of the configuration, so is the order).
 template <int NT, bool LO>
-__global__ void __launch_bounds__(kFThreads, 2) tersoff_force(const JobView* __restrict__ jobs,
+__global__ void __launch_bounds__(kFThreadsLarge, 2) tersoff_force(const JobView* __restrict__ jobs,
                                                               const WorkItem* __restrict__ items) {
   extern __shared__ __align__(16) unsigned char smem[];
   const WorkItem it = items[blockIdx.x];
   const JobView& J = jobs[it.job];
   const TersoffForceView& v = J.tf;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int c = it.config, Na = J.v.Na[c], P = J.P;
   const int lgH = v.lgH[c], H = 1 << lgH, A = 32 >> lgH;
   const int h = lane & (H - 1), aslot = lane >> lgH;
   const int base = v.base[c], n_inner = v.inner[c];
   f2* tab = reinterpret_cast<f2*>(smem);       // [FK_COUNT][H]
   f2* scratch = tab + FK_COUNT * 16;           // [slot][atom][H] records of 3
-  for (int t = threadIdx.x; t < FK_COUNT * H; t += kFThreads) {
+  for (int t = threadIdx.x; t < FK_COUNT * H; t += blockDim.x) {
     const int k = t >> lgH, hh = t & (H - 1);
     auto value = [&](int half) -> float {
       const int p = min(it.p0 + 2 * hh + half, P - 1);
@@ -331,7 +334,7 @@ __global__ void __launch_bounds__(kFThreads, 2) tersoff_force(const JobView* __r
   const float4* gu = v.gu + base;
   const float4* gd = v.gd + base;
   f2* rec = scratch + 3 * h;
-  for (int il = warp * A + aslot; il < Na; il += kFWarps * A) {
+  for (int il = warp * A + aslot; il < Na; il += warps * A) {
     if (il < n_inner) atom_forces<NT, LO, true>(K, gu, gd, Na, il, rec, lgH);
     else atom_forces<NT, LO, false>(K, gu, gd, Na, il, rec, lgH);
   }
@@ -340,7 +343,7 @@ __global__ void __launch_bounds__(kFThreads, 2) tersoff_force(const JobView* __r
   const double* ref = v.ref + (size_t)3 * (base / 4);
   double e0 = 0.0, e1 = 0.0;
   const f2 m1 = dup(-1.0f);
-  for (int il = warp * A + aslot; il < Na; il += kFWarps * A) {
+  for (int il = warp * A + aslot; il < Na; il += warps * A) {
     int rl[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) rl[j] = __ldg(rev + j * Na + il);
@@ -372,12 +375,11 @@ __global__ void __launch_bounds__(kFThreads, 2) tersoff_force(const JobView* __r
   __syncthreads();  // every f_ij has been read
   double* red = reinterpret_cast<double*>(smem);  // [half][thread]
   red[threadIdx.x] = e0;
-  red[kFThreads + threadIdx.x] = e1;
+  red[blockDim.x + threadIdx.x] = e1;
   __syncthreads();
   if (warp < 2) {
     double s = 0.0;
-#pragma unroll
-    for (int x = 0; x < kFWarps; ++x) s += red[warp * kFThreads + x * 32 + lane];
+    for (int x = 0; x < warps; ++x) s += red[warp * blockDim.x + x * 32 + lane];
     for (int o = H; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     const int p = it.p0 + 2 * lane + warp;
     if (lane < H && p < P) J.res[((size_t)p * J.v.Nc + c) * kResK + 7] = s;
@@ -385,22 +387,24 @@ __global__ void __launch_bounds__(kFThreads, 2) tersoff_force(const JobView* __r
   finish_item(jobs, it, 2 * H);
 }
 
-constexpr size_t kForceSmem = 100 * 1024;     // two CTAs per SM
+constexpr size_t kForceSmem = 52 * 1024;      // four CTAs per SM
 constexpr size_t kForceSmemMax = 200 * 1024;  // one: still better than 32 individuals with their scratch in global memory
 
 size_t force_smem(int Na, int H) {
-  return std::max((size_t)FK_COUNT * 16 * 8 + (size_t)4 * Na * H * 24, sizeof(double) * 2 * kFThreads);
+  return std::max((size_t)FK_COUNT * 16 * 8 + (size_t)4 * Na * H * 24, sizeof(double) * 2 * kFThreadsLarge);
 }
 
 }  // namespace
 
 // log2 of the pairs of individuals per item for a configuration of Na atoms (-1: too large for shared memory): the
-// largest of 16, 8, 4, 2, 1 whose scratch leaves room for two CTAs per SM.
+// largest of 16, 8, 4, 2, 1 whose scratch leaves room for four CTAs per SM, or one pair in a CTA of twice the threads (two
+// CTAs per SM: 16 warps again).
 int tersoff_force_lgH(int Na) {
   for (int l = 4; l >= 0; --l)
     if (force_smem(Na, 1 << l) <= kForceSmem) return l;
   return force_smem(Na, 1) <= kForceSmemMax ? 0 : -1;
 }
+bool tersoff_force_large(int Na) { return force_smem(Na, 1) > kForceSmem; }
 size_t tersoff_force_smem(int Na) { return force_smem(Na, 1 << tersoff_force_lgH(Na)); }
 
 int tersoff_force_build(Engine* e) {
@@ -495,7 +499,8 @@ static int force_launch(const JobView* jobs, const WorkItem* items, int count, s
     GPUGA_CUDA(cudaFuncSetAttribute(tersoff_force<NT, LO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kForceSmemMax));
     return GPUGA_OK;
   }
-  tersoff_force<NT, LO><<<count, kFThreads, smem, st>>>(jobs, items);
+  // items of the two kinds are in launches of their own
+  tersoff_force<NT, LO><<<count, smem <= kForceSmem ? kFThreads : kFThreadsLarge, smem, st>>>(jobs, items);
   GPUGA_CUDA(cudaGetLastError());
   return GPUGA_OK;
 }
