@@ -337,7 +337,10 @@ def run_ours(args, dist: Dist):
     launches = []
     for r in rows:
         items = {0: "energy_virial", 1: "force", 2: "force+energy_virial"}[int(r[2])]
-        launches.append({"kernel": f"{kinds[int(r[0])]}<{int(r[1])},{items}>",
+        kind = kinds[int(r[0])]
+        if int(r[1]) == 0:  # the classes of their own kernels
+            kind = {(0, 0): "tersoff_ev", (0, 1): "tersoff_force"}.get((int(r[0]), int(r[2])), "spectral_items")
+        launches.append({"kernel": f"{kind}<{int(r[1])},{items}>",
                          "ctas": int(r[3]), "units": r[4], "flops": r[5], "sfu_calls": r[6], "ms": r[7],
                          "tflops": (r[5] / (r[7] * 1e-3) / 1e12) if r[7] > 0 else None})
     dom = max(launches, key=lambda x: x["ms"])

@@ -63,7 +63,8 @@ typedef struct gpuga_options {
                           population plan is built, 1 the fixed rule (the largest individuals-per-item
                           count whose scratch fits shared memory), 2 half of it, 3 a quarter, 4 32
                           individuals with the scratch in global memory, 5 the fixed rule without staged
-                          geometry.  Every choice gives bit-identical results. */
+                          geometry.  Every choice gives bit-identical results.  Configurations whose
+                          atoms have at most four bonds inside fixed radii have one tile, whatever this says. */
   int fitness_fold;    /* where each individual's fitness is folded from its configurations' results:
                           0 (default) or 2 in a launch of its own after the item launches; 1 in the work
                           item that finishes the individual's last configuration (an atomic count per
@@ -141,8 +142,8 @@ int gpuga_last_config_results(gpuga_engine* e, int P, double* energy, double* vi
 int gpuga_batched_forces(gpuga_engine* e, int P, const float* pop01, float* forces_out);
 
 /* Launch plan of the batched path for population size P (built on first use).
- * *n_launches = batched launches per generation (one per kernel class: force and energy/virial items
- * share a launch, and the items fold each individual's fitness; the decode launch comes on top);
+ * *n_launches = batched launches per generation (one per kernel class; the decode launch and the fold come
+ * on top);
  * per_launch (may be NULL) receives up to `cap` rows of 8 doubles:
  * {kind (0 Tersoff, 1 RI, 2 NN2B), register class, items (0 energy/virial, 1 force, 2 both), CTAs,
  *  (individual, atom) units, algorithmic FP32 flops, transcendental calls, mean device ms per

@@ -70,3 +70,12 @@ def test_two_elements(S_free):
         data["pmin"][[3, 7]], data["pmax"][[3, 7]] = 1.5, 2.5
     data["teacher01"] = rng.uniform(0, 1, 13).astype(np.float32)
     _check(_targets(data), synth.population(data, 21, seed=4))
+
+
+@pytest.mark.parametrize("P", [1, 5])
+def test_cta_sizes(P):
+    """525 atoms are the last in a CTA of 128 threads; the two kinds of CTA in one set, and a set of the larger alone."""
+    for na in ([525, 526, 64], [526, 800]):
+        data = _cells(na + [64, 64])
+        data["Nc_force"] = len(na)
+        _check(_targets(data), synth.population(data, P, seed=10 + P))
