@@ -1,0 +1,86 @@
+// An entry of the bond-order table of tersoff_ev.cu: b(s) = (1 + (beta s)^n)^(-1/2n) and b'(s) over an interval of
+// s as one polynomial of degree 6, b = b0 + t (k0 + t (k1 + ...)), t = s - c.
+//
+// b' is what the polynomial is fitted to (degree 5 through six Chebyshev nodes), b its integral from the exact b(c):
+// a polynomial through values of b has an error in b' that is 36 times its own at the ends of the interval.
+// Which entries represent the function is decided where the error of such an interpolant has its extremes and no node
+// lies, at both ends: even and odd terms of what is left out add up at one of them, so no single coefficient that
+// happens to be zero can hide the rest.
+//
+// Bounds for an entry that is accepted (tests/test_bond_table_cpu.py; n from 0.3 to 50): b to 7e-8 of its size, b' to
+// 2e-7 of the entry's largest, or of 1e-3 / s where that is larger.  Of that 4e-8 may be the interpolation's; the rest
+// is the rounding of the FP32 coefficients and of their evaluation.  On eighths of octaves every entry is accepted for
+// n up to 5 (interpolation: 4e-9 for n up to 3); of those with beta s between 0.05 and 8 all but 6 % at n = 8, 15 % at
+// n = 12, 18 % at n = 18.
+#pragma once
+#include <cmath>
+
+#include "exp_d.cuh"
+
+#ifndef __CUDACC__
+#define GPUGA_BT_HD inline
+#else
+#define GPUGA_BT_HD __host__ __device__ __forceinline__
+#endif
+
+namespace gpuga {
+
+struct BondEntry {
+  float b0, b0lo, k[6];  // b0: b(c) and its remainder
+  bool ok;
+};
+
+// b and db/ds in closed form at s = e^ls; mh = -1/(2n), lbeta = ln beta.  b = 1, b' = 0 below beta s = 1e-16
+// (minimal_tersoff.cu:178-185).
+GPUGA_BT_HD void bond_order(double n, double mh, double beta, double lbeta, double s, double ls, double& b, double& db) {
+  const double z = n * (lbeta + ls);
+  const bool big = z > 40.0, tiny = beta * s < 1e-16;  // big: 1 + e^z = e^z
+  const double e = big ? 1.0 : exp_d_clamped(z);
+  const double v = exp_d_clamped(mh * (big ? z : log(1.0 + e)));
+  const double d = -0.5 * v * e / (big ? s : s * (1.0 + e));
+  b = tiny ? 1.0 : v;
+  db = tiny ? 0.0 : d;
+}
+
+// Where an entry is evaluated, in half widths from its center: six Chebyshev nodes, the center, both ends.
+constexpr int kBondPoints = 9, kBondCenter = 6;
+constexpr double kBondPoint[kBondPoints] = {0.96592582628906829,  0.70710678118654752,  0.25881904510252076, -0.25881904510252076,
+                                            -0.70710678118654752, -0.96592582628906829, 0.0,                 -1.0, 1.0};
+
+// The entry c - h .. c + h from h b' at those points (f) and b(c).
+GPUGA_BT_HD BondEntry bond_fit(const double (&f)[kBondPoints], double bc, double c, double h) {
+  constexpr double x[3] = {0.96592582628906829, 0.70710678118654752, 0.25881904510252076};
+  double top = 0.0;
+  for (int m = 0; m < 6; ++m) top = fmax(top, fabs(f[m]));
+  // Chebyshev coefficients (T_k at the nodes: cos(k pi (2m + 1) / 12)), then powers of t / h
+  const double e0 = f[0] + f[5], e1 = f[1] + f[4], e2 = f[2] + f[3];
+  const double o0 = f[0] - f[5], o1 = f[1] - f[4], o2 = f[2] - f[3];
+  const double a0 = (e0 + e1 + e2) / 6.0;
+  const double a1 = (o0 * x[0] + o1 * x[1] + o2 * x[2]) / 3.0;
+  const double a2 = (e0 - e2) * (0.86602540378443865 / 3.0);
+  const double a3 = (o0 - o1 - o2) * (0.70710678118654752 / 3.0);
+  const double a4 = (0.5 * e0 - e1 + 0.5 * e2) / 3.0;
+  const double a5 = (o0 * x[2] - o1 * x[1] + o2 * x[0]) / 3.0;
+  const double p[6] = {a0 - a2 + a4, a1 - 3.0 * a3 + 5.0 * a5, 2.0 * a2 - 8.0 * a4, 4.0 * a3 - 20.0 * a5, 8.0 * a4,
+                       16.0 * a5};
+  const double even = p[0] + p[2] + p[4], odd = p[1] + p[3] + p[5];
+  const double left = fmax(fabs(even + odd - f[8]), fabs(even - odd - f[7]));
+  BondEntry o;
+  o.ok = left <= 4e-8 * fmax(top, 1e-3 * h / c);  // (a NaN is not)
+  o.b0 = (float)bc;
+  o.b0lo = (float)(bc - (double)o.b0);
+  const double ih = 1.0 / h;
+  double s = ih;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+  for (int j = 0; j < 6; ++j) {
+    const double k = p[j] * s / (j + 1);
+    o.k[j] = (float)k;
+    o.ok = o.ok && fabs(k) <= 1e37;  // (intervals near s = 0: beyond FP32)
+    s *= ih;
+  }
+  return o;
+}
+
+}  // namespace gpuga

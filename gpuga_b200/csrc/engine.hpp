@@ -99,6 +99,7 @@ struct TersoffEvView {
   const int* seg0;       // [Nc + 1] first row of `part` of each configuration
   float h0;
   int tab_base, tab_n;   // b(s): first entry (top 12 bits of the FP32 s) and entries
+  const double2* points; // [tab_n][9] s and ln s where the entries are evaluated (bond_table.cuh)
   int exp_base, exp_n, n_exp;  // exponentials: first grid point, grid points, tables
   int n_part, n_items;   // items per group of 32 individuals
   // per plan

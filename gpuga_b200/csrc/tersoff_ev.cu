@@ -13,8 +13,8 @@
 // pair) is twice s, b and b', the pair terms once and 30 FMAs for W: no loop over triplets, and the same work for
 // any number of neighbors.
 //
-// b and b' come from a table per individual, polynomials of degree 5 on eighths of octaves of s: b0 (a float and
-// its remainder) + t (c1 + ...), t = s - s_c exact, so b is rounded once (5.9e-8 relative; powf_dd, which it
+// b and b' come from a table per individual, polynomials of degree 6 on eighths of octaves of s (bond_table.cuh): b0 (a
+// float and its remainder) + t (c1 + ...), t = s - s_c exact, so b is rounded once (5.9e-8 relative; powf_dd, which it
 // replaces, 6.2e-8) and b' to 2e-7.  The FP64 pair exponentials come from a table on a 1/32 A grid and a
 // degree-5 polynomial of the rest (3e-11).  Tables are per individual, lane-private in shared memory (no bank
 // conflicts whatever a lane's index) and rebuilt each generation (tersoff_tables).  s outside the table, or an
@@ -25,6 +25,7 @@
 
 #include <cuda_pipeline.h>
 
+#include "bond_table.cuh"
 #include "decode.cuh"
 #include "engine.hpp"
 #include "fold.cuh"
@@ -177,13 +178,19 @@ __global__ void ev_batches(int n, const int* __restrict__ last, EvPair* __restri
 }
 
 // ------------------------------------------------------------------------------ tables
-// One thread per (individual, entry): b at six Chebyshev nodes of the entry in FP64, the polynomial through them
-// in powers of t = s - s_c, and whether that is exact enough; then the exponentials and the constants.
-__global__ void __launch_bounds__(256) tersoff_tables(const JobView* __restrict__ jobs, const int2* __restrict__ groups) {
+// One CTA per (group of 32 individuals, entry of b): a warp per point of the entry (a chain of some 100 dependent FP64
+// operations each), then the polynomials of b and b' (bond_table.cuh) by one of them, NaN where they are not exact enough.
+// The last CTAs of a group hold its exponentials, one per warp, and the constants.
+constexpr int kTabThreads = 32 * kBondPoints;
+__host__ __device__ inline int tab_ctas(const TersoffEvView& v) {
+  return v.tab_n + (v.n_exp * v.exp_n + kBondPoints) / kBondPoints;
+}
+__global__ void __launch_bounds__(kTabThreads) tersoff_tables(const JobView* __restrict__ jobs, const int2* __restrict__ groups) {
   const int2 jg = groups[blockIdx.x];
   const JobView& J = jobs[jg.x];
   const TersoffEvView& v = J.ev;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = 8 * gridDim.y;
+  if ((int)blockIdx.y >= tab_ctas(v)) return;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int p = jg.y * 32 + lane < J.P ? jg.y * 32 + lane : J.P - 1;  // lanes without an individual repeat the last
   auto par = [&](int m) { return (double)decode1(J.pmin[m], J.pmax[m], J.pop[(size_t)p * J.num_vars + m]); };
   unsigned char* tab = v.tables + (size_t)jg.y * tab_bytes(v);
@@ -191,69 +198,47 @@ __global__ void __launch_bounds__(256) tersoff_tables(const JobView* __restrict_
   double* te = reinterpret_cast<double*>(tab + tab_b_bytes(v));
   double* tk = te + (size_t)v.n_exp * v.exp_n * 32;
   const int off = J.num_types == 2 ? 4 : 0;
-  const double n = par(4 + off), beta = par(5 + off);
-  const double lbeta = log(beta), mh = -0.5 / n;
-  auto b_of = [&](double s) {
-    if (beta * s < 1e-16) return 1.0;  // minimal_tersoff.cu:178-185
-    return exp(mh * log1p(exp(n * (lbeta + log(s)))));
-  };
-  const int total = v.tab_n + v.n_exp * v.exp_n + 1;
-  for (int i = blockIdx.y * 8 + warp; i < total; i += nwarps) {
-    if (i < v.tab_n) {
-      const double c = entry_center(i, v.tab_base), lo = (double)__int_as_float((i + v.tab_base) << 20), h = c - lo;
-      // interpolation in x = t / h at the nodes cos(pi (m + 1/2) / 6): Chebyshev coefficients, then powers
-      constexpr double x[3] = {0.96592582628906829, 0.70710678118654752, 0.25881904510252076};
-      double f[6];
+  const float nan = __int_as_float(0x7fc00000);
+  if ((int)blockIdx.y < v.tab_n) {
+    __shared__ double at[kBondPoints + 1][32];
+    const int i = blockIdx.y;
+    const double n = par(4 + off), beta = par(5 + off);
+    const double c = entry_center(i, v.tab_base), h = c - (double)__int_as_float((i + v.tab_base) << 20);
+    const double2 x = v.points[(size_t)i * kBondPoints + warp];
+    double b, db;
+    bond_order(n, -0.5 / n, beta, log(beta), x.x, x.y, b, db);
+    at[warp][lane] = h * db;
+    if (warp == kBondCenter) at[kBondPoints][lane] = b;
+    __syncthreads();
+    if (warp > 0) return;
+    double f[kBondPoints];
 #pragma unroll
-      for (int m = 0; m < 3; ++m) {
-        f[m] = b_of(c + h * x[m]);
-        f[5 - m] = b_of(c - h * x[m]);
-      }
-      // T_k at the nodes: cos(k pi (2m + 1) / 12)
-      const double e0 = f[0] + f[5], e1 = f[1] + f[4], e2 = f[2] + f[3];
-      const double o0 = f[0] - f[5], o1 = f[1] - f[4], o2 = f[2] - f[3];
-      const double a0 = (e0 + e1 + e2) / 6.0;
-      const double a1 = (o0 * x[0] + o1 * x[1] + o2 * x[2]) / 3.0;
-      const double a2 = (e0 * 0.86602540378443865 - e2 * 0.86602540378443865) / 3.0;
-      const double a3 = (o0 - o1 - o2) * 0.70710678118654752 / 3.0;
-      const double a4 = (0.5 * e0 - e1 + 0.5 * e2) / 3.0;
-      const double a5 = (o0 * x[2] - o1 * x[1] + o2 * x[0]) / 3.0;
-      const double ih = 1.0 / h;
-      double k[6];
-      k[0] = a0 - a2 + a4;
-      k[1] = (a1 - 3.0 * a3 + 5.0 * a5) * ih;
-      k[2] = (2.0 * a2 - 8.0 * a4) * ih * ih;
-      k[3] = (4.0 * a3 - 20.0 * a5) * ih * ih * ih;
-      k[4] = 8.0 * a4 * ih * ih * ih * ih;
-      k[5] = 16.0 * a5 * ih * ih * ih * ih * ih;
-      const float b0 = (float)k[0];
-      // the degree-5 term against the fall of the coefficients bounds what is left out: b to 3e-9, and t b' (whose
-      // series loses a factor 5) to 1e-7 of its own size
-      const double left = fabs(a5) * fmin(1.0, fabs(a5) / fmax(fabs(a4), 1e-300));
-      const bool ok = left <= 3e-9 && 36.0 * left <= 2e-7 * (fabs(a1) * 16.0 + 0.01);
-      const float nan = __int_as_float(0x7fc00000);  // not represented: taken as outside the table
-      ta[i * 64 + lane] = make_float4(ok ? b0 : nan, (float)(k[0] - (double)b0), (float)k[1], (float)k[2]);
-      ta[i * 64 + 32 + lane] = make_float4((float)k[3], (float)k[4], (float)k[5], 0.f);
-    } else if (i < v.tab_n + v.n_exp * v.exp_n) {
-      const int k = i - v.tab_n, which = k / v.exp_n, e = k - which * v.exp_n;
-      // exponentials in the order la, lr (S not fixed at 2) of set 0, then of set 1
-      const int per = v.n_exp / J.num_types, s = which / per, q = J.num_types == 2 && s == 1 ? 4 : 0;
-      const double A = par(q + 1), R0 = par(q + 2), S = par(q + 3);
-      const double l = which % per ? sqrt(2.0 * S) * A : sqrt(2.0 / S) * A;
-      te[(size_t)k * 32 + lane] = exp(-l * ((e + v.exp_base) * kStep - R0));
-    } else {
-      for (int s = 0; s < J.num_types; ++s) {
-        const int q = 4 * s;
-        const double D0 = par(q + 0), A = par(q + 1), S = par(q + 3);
-        tk[(4 * s + 0) * 32 + lane] = sqrt(2.0 / S) * A;
-        tk[(4 * s + 1) * 32 + lane] = S * D0 / (S - 1.0);
-        tk[(4 * s + 2) * 32 + lane] = sqrt(2.0 * S) * A;
-        tk[(4 * s + 3) * 32 + lane] = D0 / (S - 1.0);
-      }
-      tk[8 * 32 + lane] = par(6 + off) - (double)v.h0;
-      const float nan = __int_as_float(0x7fc00000);
-      ta[v.tab_n * 64 + lane] = ta[v.tab_n * 64 + 32 + lane] = make_float4(nan, nan, nan, nan);
+    for (int k = 0; k < kBondPoints; ++k) f[k] = at[k][lane];
+    const BondEntry e = bond_fit(f, at[kBondPoints][lane], c, h);
+    // not represented: taken as outside the table
+    ta[i * 64 + lane] = make_float4(e.ok ? e.b0 : nan, e.b0lo, e.k[0], e.k[1]);
+    ta[i * 64 + 32 + lane] = make_float4(e.k[2], e.k[3], e.k[4], e.k[5]);
+    return;
+  }
+  const int k = (blockIdx.y - v.tab_n) * kBondPoints + warp;
+  if (k < v.n_exp * v.exp_n) {
+    const int which = k / v.exp_n, e = k - which * v.exp_n;
+    // exponentials in the order la, lr (S not fixed at 2) of set 0, then of set 1
+    const int per = v.n_exp / J.num_types, s = which / per, q = J.num_types == 2 && s == 1 ? 4 : 0;
+    const double A = par(q + 1), R0 = par(q + 2), S = par(q + 3);
+    const double l = which % per ? sqrt(2.0 * S) * A : sqrt(2.0 / S) * A;
+    te[(size_t)k * 32 + lane] = exp(-l * ((e + v.exp_base) * kStep - R0));
+  } else if (k == v.n_exp * v.exp_n) {
+    for (int s = 0; s < J.num_types; ++s) {
+      const int q = 4 * s;
+      const double D0 = par(q + 0), A = par(q + 1), S = par(q + 3);
+      tk[(4 * s + 0) * 32 + lane] = sqrt(2.0 / S) * A;
+      tk[(4 * s + 1) * 32 + lane] = S * D0 / (S - 1.0);
+      tk[(4 * s + 2) * 32 + lane] = sqrt(2.0 * S) * A;
+      tk[(4 * s + 3) * 32 + lane] = D0 / (S - 1.0);
     }
+    tk[8 * 32 + lane] = par(6 + off) - (double)v.h0;
+    ta[v.tab_n * 64 + lane] = ta[v.tab_n * 64 + 32 + lane] = make_float4(nan, nan, nan, nan);
   }
 }
 
@@ -297,7 +282,9 @@ __device__ __forceinline__ void ev_pairs_of(const EvLane<NT, LO>& L, const EvPai
         const unsigned i = min((unsigned)((bits >> 20) - L.tab_base), (unsigned)L.tab_n);
         const float4 k0 = L.ta[i * 64], k1 = L.ta[i * 64 + 32];
         const float t = s - __int_as_float((bits & 0xfff00000) | 0x00080000);
-        float pl = fmaf(k1.z, t, k1.y), d = fmaf(k1.z, t, pl);
+        float pl = fmaf(k1.w, t, k1.z), d = fmaf(k1.w, t, pl);
+        pl = fmaf(pl, t, k1.y);
+        d = fmaf(d, t, pl);
         pl = fmaf(pl, t, k1.x);
         d = fmaf(d, t, pl);
         pl = fmaf(pl, t, k0.w);
@@ -579,12 +566,26 @@ int tersoff_ev_build(Engine* e) {
     const int top = entry(smax * 1.0001), low = std::max(entry(smin * 0.9999), top - kTabMax + 1);
     v.tab_base = low;
     v.tab_n = top - low + 1;
+    std::vector<double2> points((size_t)v.tab_n * kBondPoints);
+    for (int k = 0; k < v.tab_n; ++k) {
+      const int32_t lo = (low + k) << 20, mid = lo | 0x00080000;
+      float f, c;
+      memcpy(&f, &lo, 4);
+      memcpy(&c, &mid, 4);
+      for (int x = 0; x < kBondPoints; ++x) {
+        const double s = c + ((double)c - f) * kBondPoint[x];
+        points[(size_t)k * kBondPoints + x] = make_double2(s, std::log(s));
+      }
+    }
     bool exact = true;  // S fixed at 2: one exponential per bond (tersoff_consts_exact)
     for (int s = 0; s < d.num_types; ++s) exact &= sp.pmin[4 * s + 3] == 2.0f && sp.pmax[4 * s + 3] == 2.0f;
     v.n_exp = d.num_types * (exact ? 1 : 2);
     if (tersoff_ev_smem(v) > 220 * 1024) return GPUGA_OK;
     TersoffSegment* d_segs = nullptr;
     int* d_seg0 = nullptr;
+    double2* d_points = nullptr;
+    GPUGA_TRY(e->alloc(&d_points, points.size()));
+    GPUGA_CUDA(cudaMemcpy(d_points, points.data(), sizeof(double2) * points.size(), cudaMemcpyHostToDevice));
     GPUGA_TRY(e->alloc(&d_segs, segs.size()));
     GPUGA_TRY(e->alloc(&d_seg0, seg0.size()));
     GPUGA_CUDA(cudaMemcpy(d_segs, segs.data(), sizeof(TersoffSegment) * segs.size(), cudaMemcpyHostToDevice));
@@ -604,6 +605,7 @@ int tersoff_ev_build(Engine* e) {
     v.pairs = pairs;
     v.shell = shell;
     v.segs = d_segs;
+    v.points = d_points;
     v.seg0 = d_seg0;
     v.n_part = parts;
     v.n_items = (int)e->h_ev_items.size();
@@ -631,8 +633,10 @@ int tersoff_ev_plan(Engine* e, Plan* plan) {
 }
 
 int tersoff_tables_launch(const LaunchSet* ls, cudaStream_t st) {
-  // enough warps for an entry each: the FP64 chains of an entry take about 10 us
-  tersoff_tables<<<dim3(ls->ev_groups, 16), 256, 0, st>>>(ls->d_jobs, ls->d_evgroups);
+  int ctas = 0;  // of a group, of the job with most
+  for (const JobView& j : ls->jobs)
+    if (j.ev.pairs) ctas = std::max(ctas, tab_ctas(j.ev));
+  tersoff_tables<<<dim3(ls->ev_groups, ctas), kTabThreads, 0, st>>>(ls->d_jobs, ls->d_evgroups);
   GPUGA_CUDA(cudaGetLastError());
   return GPUGA_OK;
 }
