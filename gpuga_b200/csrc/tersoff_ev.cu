@@ -300,6 +300,9 @@ __device__ __forceinline__ void ev_pairs_of(const EvLane<NT, LO>& L, const EvPai
         if (zeta < 1.0e-16f) {
           bo[h] = 1.f;
           db[h] = 0.f;
+        } else if (zn > 1.0e30f) {  // 1 + zeta^n = zeta^n, which may be beyond FP32
+          bo[h] = powf_dd(zeta, -0.5f);
+          db[h] = -0.5f * bo[h] / s;
         }
       }
     }

@@ -96,8 +96,8 @@ def _check(data, pop):
                 assert np.abs(W[p, c] - w[:, a:b].sum(1)).max() <= tol
 
 
-@pytest.mark.parametrize("n,closed", [(0.787, True), (0.787, False), (3, True), (3, False), (6, True), (6, False),
-                                      (12, True), (12, False), (22.956, True), (22.956, False), (50, True)])
+@pytest.mark.parametrize("closed", [True, False])
+@pytest.mark.parametrize("n", [0.787, 3, 6, 12, 22.956, 50])
 def test_bond_orders_one_by_one(n, closed):
     """beta s from below to above 1, where b bends."""
     data = _trimers({4: (0.97 * n, 1.03 * n), 5: (0.2, 2) if closed else (2, 20)}, closed)
