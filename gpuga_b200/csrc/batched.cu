@@ -1474,7 +1474,7 @@ struct ItemSpec {
   double cost, units, flops, sfu;
 };
 struct LaunchKey {
-  int kind, zclass, nmax, force, lo, expansion;  // expansion: 1 pair expansion or Tersoff pairs, 2, 3 packed Tersoff forces (two sizes of CTA)
+  int kind, zclass, nmax, force, lo, expansion;  // expansion: 1 pair expansion or Tersoff pairs, 2, 3 packed Tersoff forces (two sizes of CTA), 4 Tersoff pairs, wide
   bool operator<(const LaunchKey& o) const {
     return std::tie(kind, zclass, nmax, force, lo, expansion) <
            std::tie(o.kind, o.zclass, o.nmax, o.force, o.lo, o.expansion);
@@ -1686,7 +1686,7 @@ int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<I
     }
   }
   if (d.ev.pairs && !only) {
-    const LaunchKey key{0, 0, nmax, 0, lo ? 1 : 0, 1};
+    const LaunchKey key{0, 0, nmax, 0, lo ? 1 : 0, d.ev.wide ? 4 : 1};
     smem_need[key] = std::max(smem_need[key], tersoff_ev_smem(d.ev));
     for (const EvItem& x : e->h_ev_items)
       for (int p0 = 0; p0 < P; p0 += 32) {
@@ -1735,7 +1735,8 @@ int launch_one(const LaunchSet* ls, const Launch& L, cudaStream_t st, bool confi
   const WorkItem* items = ls->d_items + L.first;
   if (L.packed) return tersoff_force_launch(ls->d_jobs, items, L.count, L.smem, L.nmax, L.lo, configure_only, st);
   if (L.expansion && L.kind == 0)
-    return tersoff_ev_items_launch(ls->d_jobs, items, L.count, L.smem, L.nmax, L.lo, configure_only, st);
+    return tersoff_ev_items_launch(ls->d_jobs, items, L.count, L.smem, L.nmax, L.lo, L.wide, configure_only,
+                                   st);
   if (L.expansion) return configure_only ? GPUGA_OK : spectral_items_launch(ls->d_jobs, items, L.count, st);
 #define GPUGA_TERSOFF1(ZC, NT)                                                          \
   do {                                                                                  \
@@ -1853,8 +1854,9 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
     L.zclass = kv.first.zclass;
     L.nmax = kv.first.nmax;
     L.lo = kv.first.lo != 0;
-    L.expansion = kv.first.expansion == 1;
-    L.packed = kv.first.expansion >= 2;
+    L.wide = kv.first.expansion == 4;
+    L.expansion = kv.first.expansion == 1 || L.wide;
+    L.packed = kv.first.expansion == 2 || kv.first.expansion == 3;
     L.fallback = L.kind != 0 && !L.expansion && !plain_pairs[L.kind];
     int nforce = 0;
     for (auto& t : v) nforce += item_force(t.w) ? 1 : 0;

@@ -101,6 +101,7 @@ struct TersoffEvView {
   int tab_base, tab_n;   // b(s): first entry (top 12 bits of the FP32 s) and entries
   const double2* points; // [tab_n][9] s and ln s where the entries are evaluated (bond_table.cuh)
   int exp_base, exp_n, n_exp;  // exponentials: first grid point, grid points, tables
+  bool wide;             // the form for sharp n and steep exponentials
   int n_part, n_items;   // items per group of 32 individuals
   // per plan
   unsigned char* tables; // [individuals / 32]
@@ -257,6 +258,7 @@ struct Launch {
   int kind = 0;        // 0 Tersoff, 1 RI, 2 NN2B
   bool expansion = false;  // items of the pair expansion (spectral.cu), Tersoff: of pairs (tersoff_ev.cu)
   bool packed = false;     // packed Tersoff force items (tersoff_force.cu)
+  bool wide = false;       // Tersoff pairs: the form for sharp n and steep exponentials (tersoff_ev.cu)
   bool fallback = false;   // RI / NN2B direct items that only take the individuals the expansion left
   int zclass = 4;      // Tersoff register-array size
   int nmax = 0;        // NN2B register-array size; Tersoff: number of atom types
@@ -396,7 +398,7 @@ size_t tersoff_ev_smem(const TersoffEvView& v);
 size_t tersoff_ev_table_bytes(const TersoffEvView& v);
 int tersoff_tables_launch(const LaunchSet* ls, cudaStream_t st);  // tables and decode
 int tersoff_ev_items_launch(const JobView* jobs, const WorkItem* items, int count, size_t smem, int num_types, bool lo,
-                            bool configure, cudaStream_t st);
+                            bool wide, bool configure, cudaStream_t st);
 
 // tersoff_force.cu
 int tersoff_force_build(Engine* e);

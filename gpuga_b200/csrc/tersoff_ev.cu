@@ -15,10 +15,17 @@
 //
 // b and b' come from a table per individual, polynomials of degree 6 on eighths of octaves of s (bond_table.cuh): b0 (a
 // float and its remainder) + t (c1 + ...), t = s - s_c exact, so b is rounded once (5.9e-8 relative; powf_dd, which it
-// replaces, 6.2e-8) and b' to 2e-7.  The FP64 pair exponentials come from a table on a 1/32 A grid and a
-// degree-5 polynomial of the rest (3e-11).  Tables are per individual, lane-private in shared memory (no bank
-// conflicts whatever a lane's index) and rebuilt each generation (tersoff_tables).  s outside the table, or an
-// individual whose n is too sharp for it (checked when it is built), takes powf_dd.
+// replaces, 6.2e-8) and b' to 2e-7.  The FP64 pair exponentials e^{-l t} come from a table on a 1/32 A grid and a
+// polynomial of the rest, |l delta| <= l / 64, of degree m, which leaves out (l / 64)^(m + 1) / (m + 1)!: 3e-11 for m = 5 up
+// to l = 3.38 A^-1 (alpha 1.5 with S 2.5) and for m = 9 up to 25.  Tables are per individual, lane-private in shared
+// memory (no bank conflicts whatever a lane's index) and rebuilt each generation (tersoff_tables).  s outside the table,
+// an individual whose n is too sharp for it (checked when it is built) or whose l is beyond the polynomial takes powf_dd
+// and exp_d.
+//
+// Two forms of the items, by the bounds (TersoffEvView::wide).  The plain one has m = 5 and evaluates a batch that needs
+// powf_dd a second time; where l may be above 3.38 or n above 5, m = 9, and powf_dd bond by bond: 67 configurations of up
+// to 1000 atoms at population 333 with n from 8 to 12 and beta s around 1, 394 us a generation (530 in the plain
+// form, 458 by atom), but 202 against 192 us for n below 0.8.  A set that allows l above 25 stays with the items by atom.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -28,6 +35,7 @@
 #include "bond_table.cuh"
 #include "decode.cuh"
 #include "engine.hpp"
+#include "exp_d.cuh"
 #include "fold.cuh"
 #include "powf_dd.cuh"
 
@@ -41,6 +49,7 @@ constexpr int kEvConsts = 10;         // doubles per individual: la, ca, lr, cr 
 constexpr int kSetBit = 1 << 16, kShellBit = 1 << 17;  // EvPair::code: pair set; a neighbor lies in R1 .. R2 (of any pair of the batch)
 constexpr int kTabMax = 80, kExpMax = 96;
 constexpr double kStep = 1.0 / 32.0;  // distance grid
+constexpr double kExpFlat = 3.38, kExpSteep = 25.0;  // steepest exponential of the two polynomials, 1 / A
 
 // bytes of an individual group's tables (32 lanes): b as two float4 per entry (the last entry, NaN, stands for
 // every s outside the table), exponentials, constants
@@ -227,7 +236,8 @@ __global__ void __launch_bounds__(kTabThreads) tersoff_tables(const JobView* __r
     const int per = v.n_exp / J.num_types, s = which / per, q = J.num_types == 2 && s == 1 ? 4 : 0;
     const double A = par(q + 1), R0 = par(q + 2), S = par(q + 3);
     const double l = which % per ? sqrt(2.0 * S) * A : sqrt(2.0 / S) * A;
-    te[(size_t)k * 32 + lane] = exp(-l * ((e + v.exp_base) * kStep - R0));
+    const double value = exp(-l * ((e + v.exp_base) * kStep - R0));
+    te[(size_t)k * 32 + lane] = fabs(l) <= (v.wide ? kExpSteep : kExpFlat) ? value : (double)nan;  // NaN: the exact form
   } else if (k == v.n_exp * v.exp_n) {
     for (int s = 0; s < J.num_types; ++s) {
       const int q = 4 * s;
@@ -243,7 +253,8 @@ __global__ void __launch_bounds__(kTabThreads) tersoff_tables(const JobView* __r
 }
 
 // ------------------------------------------------------------------------------ items
-// NT: atom types; LO: S is a fitted parameter (two exponentials per pair; else lr = 2 la and cr = ca / 2).
+// NT: atom types; LO: S is a fitted parameter (two exponentials per pair; else lr = 2 la and cr = ca / 2); WIDE: see
+// above.
 // One CTA: the segments of the item (up to kEvSegPairs pairs of one configuration each) for 32 individuals, a lane
 // each; the warps take batches of 2 consecutive pairs in turn, whose coefficients come through a two-stage
 // buffer per warp (cp.async), E summed in FP64, W in FP32 over a batch and in FP64 beyond.
@@ -262,48 +273,77 @@ struct EvLane {
   int tab_base, tab_n, exp_base, exp_n;
 };
 
-// The pairs of a batch.  EXACT: b and b' by powf_dd (a bond of the batch lies outside the table).
-template <int NT, bool LO, bool EXACT>
+// b and b' by powf_dd (rare; out of line, so that its registers do not count).
+__device__ __noinline__ float2 bond_exact(float s, float beta, float n, float mhon, float mhonl) {
+  const float zeta = beta * s;
+  if (zeta < 1.0e-16f) return make_float2(1.f, 0.f);
+  const float zn = powf_dd(zeta, n), opz = 1.0f + zn;
+  if (zn > 1.0e30f) {  // 1 + zeta^n = zeta^n, which may be beyond FP32
+    const float b = powf_dd(zeta, -0.5f);
+    return make_float2(b, -0.5f * b / s);
+  }
+  const float b = powf_dd(opz, mhon, mhonl);
+  return make_float2(b, beta * __fdividef(-0.5f * b * zn, opz * zeta));
+}
+
+// The pairs of a batch.  WIDE: bonds outside the table take bond_exact one by one, before the pair terms; else EXACT, a
+// second pass for all bonds of the batch.  EXACT: also exp_d where the exponentials lie outside the table.
+template <int NT, bool LO, bool WIDE, bool EXACT>
 __device__ __forceinline__ void ev_pairs_of(const EvLane<NT, LO>& L, const EvPair* q, const float4* x2, const Consts& kc,
                                             double& E, float (&w)[6]) {
   float Qh[kEvBatch][2];
+  float bo[kEvBatch][2], db[kEvBatch][2];  // b(s), b'(s)
+  auto exact = [&](int u, int h, float s) {
+    const float2 r = bond_exact(s, kc[TC_BETA], kc[TC_EN], kc[TC_MHON], kc[TC_MHONL]);
+    bo[u][h] = r.x;
+    db[u][h] = r.y;
+  };
+  auto table = [&](int u, int h, float s) {
+    const int bits = __float_as_int(s);
+    const unsigned i = min((unsigned)((bits >> 20) - L.tab_base), (unsigned)L.tab_n);
+    const float4 k0 = L.ta[i * 64], k1 = L.ta[i * 64 + 32];
+    const float t = s - __int_as_float((bits & 0xfff00000) | 0x00080000);
+    float pl = fmaf(k1.w, t, k1.z), d = fmaf(k1.w, t, pl);
+    pl = fmaf(pl, t, k1.y);
+    d = fmaf(d, t, pl);
+    pl = fmaf(pl, t, k1.x);
+    d = fmaf(d, t, pl);
+    pl = fmaf(pl, t, k0.w);
+    d = fmaf(d, t, pl);
+    pl = fmaf(pl, t, k0.z);
+    db[u][h] = fmaf(d, t, pl);
+    bo[u][h] = k0.x + fmaf(pl, t, k0.y);
+  };
+  if constexpr (WIDE) {
+    auto s_of = [&](int u, int h) { return (float)fma(L.dh, fma(L.dh, q[u].C[h], q[u].B[h]), q[u].A[h]); };
+    bool outside = false;
+#pragma unroll
+    for (int u = 0; u < kEvBatch; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        table(u, h, s_of(u, h));
+        outside |= bo[u][h] != bo[u][h];
+      }
+    if (__any_sync(0xffffffffu, outside)) {
+#pragma unroll
+      for (int u = 0; u < kEvBatch; ++u)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+          if (bo[u][h] != bo[u][h]) exact(u, h, s_of(u, h));  // its lanes alone: no result depends on the group
+    }
+  }
 #pragma unroll
   for (int u = 0; u < kEvBatch; ++u) {
     const float4* f = reinterpret_cast<const float4*>(q + u);
     const double2 A = *reinterpret_cast<const double2*>(f), B = *reinterpret_cast<const double2*>(f + 1),
                   C = *reinterpret_cast<const double2*>(f + 2), f3 = *reinterpret_cast<const double2*>(f + 3);
     const float4 f4 = f[4];  // hfcp (double), hfc32, code
-    float bo[2], db[2];      // b(s), b'(s)
+    if constexpr (!WIDE) {
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float s = h == 0 ? (float)fma(L.dh, fma(L.dh, C.x, B.x), A.x) : (float)fma(L.dh, fma(L.dh, C.y, B.y), A.y);
-      if constexpr (!EXACT) {
-        const int bits = __float_as_int(s);
-        const unsigned i = min((unsigned)((bits >> 20) - L.tab_base), (unsigned)L.tab_n);
-        const float4 k0 = L.ta[i * 64], k1 = L.ta[i * 64 + 32];
-        const float t = s - __int_as_float((bits & 0xfff00000) | 0x00080000);
-        float pl = fmaf(k1.w, t, k1.z), d = fmaf(k1.w, t, pl);
-        pl = fmaf(pl, t, k1.y);
-        d = fmaf(d, t, pl);
-        pl = fmaf(pl, t, k1.x);
-        d = fmaf(d, t, pl);
-        pl = fmaf(pl, t, k0.w);
-        d = fmaf(d, t, pl);
-        pl = fmaf(pl, t, k0.z);
-        db[h] = fmaf(d, t, pl);
-        bo[h] = k0.x + fmaf(pl, t, k0.y);
-      } else {
-        const float beta = kc[TC_BETA], zeta = beta * s;
-        const float zn = powf_dd(zeta, kc[TC_EN]), opz = 1.0f + zn;
-        bo[h] = powf_dd(opz, kc[TC_MHON], kc[TC_MHONL]);
-        db[h] = beta * __fdividef(-0.5f * bo[h] * zn, opz * zeta);
-        if (zeta < 1.0e-16f) {
-          bo[h] = 1.f;
-          db[h] = 0.f;
-        } else if (zn > 1.0e30f) {  // 1 + zeta^n = zeta^n, which may be beyond FP32
-          bo[h] = powf_dd(zeta, -0.5f);
-          db[h] = -0.5f * bo[h] / s;
-        }
+      for (int h = 0; h < 2; ++h) {
+        const float s = h == 0 ? (float)fma(L.dh, fma(L.dh, C.x, B.x), A.x) : (float)fma(L.dh, fma(L.dh, C.y, B.y), A.y);
+        if constexpr (EXACT) exact(u, h, s);
+        else table(u, h, s);
       }
     }
     // pair terms: exponentials from the grid point and a polynomial of the rest
@@ -312,19 +352,25 @@ __device__ __forceinline__ void ev_pairs_of(const EvLane<NT, LO>& L, const EvPai
     const int set = NT == 2 ? (code >> 16) & 1 : 0;
     const double la = NT == 2 ? L.tk[set * 128] : L.la, ca = NT == 2 ? L.tk[set * 128 + 32] : L.ca;
     const double* tx = L.te + (size_t)((NT == 2 ? set * (LO ? 2 : 1) * L.exp_n : 0) + e) * 32;
-    auto ex = [](double y, double base) {
-      double z = fma(y, 1.0 / 120.0, 1.0 / 24.0);
-      z = fma(y, z, 1.0 / 6.0);
-      z = fma(y, z, 0.5);
-      z = fma(y, z, 1.0);
-      return fma(base * y, z, base);
+    auto ex = [&](double l, double base) {
+      const double y = -l * f3.x;
+      constexpr double inv_fact[10] = {1.0,         1.0,         0.5,          1.0 / 6.0,     1.0 / 24.0,
+                                       1.0 / 120.0, 1.0 / 720.0, 1.0 / 5040.0, 1.0 / 40320.0, 1.0 / 362880.0};
+      constexpr int deg = WIDE ? 9 : 5;
+      double z = inv_fact[deg];
+#pragma unroll
+      for (int k = deg - 1; k >= 1; --k) z = fma(y, z, inv_fact[k]);
+      double r = fma(base * y, z, base);
+      // beyond the tables: of d - r0, d = grid point + delta exactly
+      if (EXACT && r != r) r = exp_d_clamped(-l * ((code & 0xffff) * kStep + f3.x - (double)kc[TC_R0 + set]));
+      return r;
     };
-    const double ea = ex(-la * f3.x, tx[0]);
-    const double fa = ca * ea, bs = (double)bo[0] + (double)bo[1];
+    const double ea = ex(la, tx[0]);
+    const double fa = ca * ea, bs = (double)bo[u][0] + (double)bo[u][1];
     double en, dA;  // over both bonds: fr - b fa and fr' - b fa'
     if constexpr (LO) {
       const double lr = NT == 2 ? L.tk[set * 128 + 64] : L.lr, cr = NT == 2 ? L.tk[set * 128 + 96] : L.cr;
-      const double fr2 = 2.0 * cr * ex(-lr * f3.x, tx[(size_t)L.exp_n * 32]);
+      const double fr2 = 2.0 * cr * ex(lr, tx[(size_t)L.exp_n * 32]);
       en = fma(-bs, fa, fr2);
       dA = fma(bs * la, fa, -lr * fr2);
     } else {
@@ -337,7 +383,7 @@ __device__ __forceinline__ void ev_pairs_of(const EvLane<NT, LO>& L, const EvPai
     const double hfcp = __hiloint2double(__float_as_int(f4.y), __float_as_int(f4.x));
     const float g = (float)-fma(hfcp, en, f3.y * dA);  // -A'/2
     const float fw = f4.z * (float)fa;
-    const float Q0 = fw * db[0], Q1 = fw * db[1];
+    const float Q0 = fw * db[u][0], Q1 = fw * db[u][1];
     Qh[u][0] = Q0 * L.dhf;
     Qh[u][1] = Q1 * L.dhf;
     // 24 + 6 floats from f5 on: D, then X0, X1 of the first and of the second bond
@@ -365,14 +411,14 @@ __device__ __forceinline__ void ev_pairs_of(const EvLane<NT, LO>& L, const EvPai
   }
 }
 
-// A batch again without the table (rare; out of line, so that its registers do not count).
-template <int NT, bool LO>
+// A batch again with exp_d (rare; out of line, so that its registers do not count).
+template <int NT, bool LO, bool WIDE>
 __device__ __noinline__ void ev_batch_exact(const EvLane<NT, LO>& L, const EvPair* q, const float4* x2, const Consts& kc,
                                             double& E, float (&w)[6]) {
-  ev_pairs_of<NT, LO, true>(L, q, x2, kc, E, w);
+  ev_pairs_of<NT, LO, WIDE, true>(L, q, x2, kc, E, w);
 }
 
-template <int NT, bool LO>
+template <int NT, bool LO, bool WIDE>
 __global__ void __launch_bounds__(kEvThreads, 2) tersoff_ev(const JobView* __restrict__ jobs,
                                                             const WorkItem* __restrict__ items) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -407,6 +453,7 @@ __global__ void __launch_bounds__(kEvThreads, 2) tersoff_ev(const JobView* __res
   }
   L.dh = L.tk[8 * 32];
   L.dhf = (float)L.dh;
+  const Consts kc{J.consts, J.Pstride, p < J.P ? p : J.P - 1};
   for (int sg = it.config; sg < it.config + it.gofs; ++sg) {
     const TersoffSegment seg = v.segs[sg];
     double E = 0.0, Wd[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -426,14 +473,13 @@ __global__ void __launch_bounds__(kEvThreads, 2) tersoff_ev(const JobView* __res
       const float4* x2 = v.shell + 4 * (size_t)(seg.b0 + b);
       double Eb = 0.0;
       float w[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      ev_pairs_of<NT, LO, false>(L, q, x2, Consts{}, Eb, w);
-      // the table's NaN entries reach the energy: such a batch again, without the table
+      ev_pairs_of<NT, LO, WIDE, false>(L, q, x2, kc, Eb, w);
+      // the NaN of a bond order or an exponential outside the tables reaches the energy
       if (__any_sync(0xffffffffu, Eb != Eb)) {
         const EvLane<NT, LO> copy = L;  // (passed by address)
-        const Consts kc{J.consts, J.Pstride, p < J.P ? p : J.P - 1};
         double Ex = 0.0;
         float wx[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        ev_batch_exact<NT, LO>(copy, q, x2, kc, Ex, wx);
+        ev_batch_exact<NT, LO, WIDE>(copy, q, x2, kc, Ex, wx);
         if (Eb != Eb) {  // only the lanes that need it: an individual's result does not depend on its group
           Eb = Ex;
 #pragma unroll
@@ -482,9 +528,22 @@ int tersoff_ev_build(Engine* e) {
   const float r1 = sp.pmin[7 + off], r2 = sp.pmin[8 + off], hlo = sp.pmin[6 + off], hhi = sp.pmax[6 + off];
   if (sp.pmax[7 + off] != r1 || sp.pmax[8 + off] != r2 || !(r1 < r2) || !std::isfinite(hlo) || !std::isfinite(hhi))
     return GPUGA_OK;
+  bool exact = true;  // S fixed at 2: one exponential per bond (tersoff_consts_exact)
+  for (int s = 0; s < d.num_types; ++s) exact &= sp.pmin[4 * s + 3] == 2.0f && sp.pmax[4 * s + 3] == 2.0f;
+  // the steepest exponential within the bounds: sqrt(2 / S) alpha and sqrt(2 S) alpha
+  double steepest = 0.0;
+  for (int s = 0; s < d.num_types; ++s) {
+    const double al = std::max(std::fabs(sp.pmin[4 * s + 1]), std::fabs(sp.pmax[4 * s + 1]));
+    const double s0 = std::min(sp.pmin[4 * s + 3], sp.pmax[4 * s + 3]), s1 = std::max(sp.pmin[4 * s + 3], sp.pmax[4 * s + 3]);
+    if (!(s0 > 0.0)) return GPUGA_OK;
+    steepest = std::max(steepest, al * std::max(std::sqrt(2.0 / s0), exact ? 0.0 : std::sqrt(2.0 * s1)));
+  }
+  if (!(steepest <= kExpSteep)) return GPUGA_OK;
   cudaStream_t st = e->stream;
   TersoffEvView v{};
   v.h0 = 0.5f * hlo + 0.5f * hhi;
+  // n up to which every entry of the table is accepted, and the shorter polynomial's steepest exponential
+  v.wide = steepest > kExpFlat || !(std::max(sp.pmin[4 + off], sp.pmax[4 + off]) <= 5.0f);
   int *d_count = nullptr, *d_start = nullptr, *d_place = nullptr, *d_last = nullptr, *d_slot = nullptr;
   double2* d_range = nullptr;
   std::vector<int> count(na), start(na + 1, 0);
@@ -508,7 +567,7 @@ int tersoff_ev_build(Engine* e) {
         dmax = std::max(dmax, range[1 + a].y);
       }
     }
-    if (start[na] == 0 || !(dmax < 1e4)) return GPUGA_OK;
+    if (start[na] == 0 || !(dmax < 2000.0)) return GPUGA_OK;  // (EvPair::code has 16 bits for the grid point)
     // A configuration's fixed costs (two CTA barriers and the fold over the warps) outweigh its pairs below about 64:
     // sets of 8-atom cells (16 pairs) took 42-66 us by atom against 55-83 here, 64-atom cells (128 pairs)
     // 52-66 against 50-66, 216-atom ones 94-103 against 51-55.
@@ -580,8 +639,6 @@ int tersoff_ev_build(Engine* e) {
         points[(size_t)k * kBondPoints + x] = make_double2(s, std::log(s));
       }
     }
-    bool exact = true;  // S fixed at 2: one exponential per bond (tersoff_consts_exact)
-    for (int s = 0; s < d.num_types; ++s) exact &= sp.pmin[4 * s + 3] == 2.0f && sp.pmax[4 * s + 3] == 2.0f;
     v.n_exp = d.num_types * (exact ? 1 : 2);
     if (tersoff_ev_smem(v) > 220 * 1024) return GPUGA_OK;
     TersoffSegment* d_segs = nullptr;
@@ -644,24 +701,24 @@ int tersoff_tables_launch(const LaunchSet* ls, cudaStream_t st) {
   return GPUGA_OK;
 }
 
-template <int NT, bool LO>
+template <int NT, bool LO, bool WIDE>
 static int ev_launch(const JobView* jobs, const WorkItem* items, int count, size_t smem, bool configure, cudaStream_t st) {
   if (configure) {
-    GPUGA_CUDA(cudaFuncSetAttribute(tersoff_ev<NT, LO>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    GPUGA_CUDA(cudaFuncSetAttribute(tersoff_ev<NT, LO, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     return GPUGA_OK;
   }
-  tersoff_ev<NT, LO><<<count, kEvThreads, smem, st>>>(jobs, items);
+  tersoff_ev<NT, LO, WIDE><<<count, kEvThreads, smem, st>>>(jobs, items);
   GPUGA_CUDA(cudaGetLastError());
   return GPUGA_OK;
 }
 
 int tersoff_ev_items_launch(const JobView* jobs, const WorkItem* items, int count, size_t smem, int num_types, bool lo,
-                            bool configure, cudaStream_t st) {
-  if (num_types == 2)
-    return lo ? ev_launch<2, true>(jobs, items, count, smem, configure, st)
-              : ev_launch<2, false>(jobs, items, count, smem, configure, st);
-  return lo ? ev_launch<1, true>(jobs, items, count, smem, configure, st)
-            : ev_launch<1, false>(jobs, items, count, smem, configure, st);
+                            bool wide, bool configure, cudaStream_t st) {
+  auto launch = num_types == 2 ? (lo ? (wide ? ev_launch<2, true, true> : ev_launch<2, true, false>)
+                                     : (wide ? ev_launch<2, false, true> : ev_launch<2, false, false>))
+                               : (lo ? (wide ? ev_launch<1, true, true> : ev_launch<1, true, false>)
+                                     : (wide ? ev_launch<1, false, true> : ev_launch<1, false, false>));
+  return launch(jobs, items, count, smem, configure, st);
 }
 
 }  // namespace gpuga
