@@ -13,14 +13,13 @@
 // pair) is twice s, b and b', the pair terms once and 30 FMAs for W: no loop over triplets, and the same work for
 // any number of neighbors.
 //
-// b and b' come from a table per individual, polynomials of degree 6 on eighths of octaves of s (bond_table.cuh): b0 (a
-// float and its remainder) + t (c1 + ...), t = s - s_c exact, so b is rounded once (5.9e-8 relative; powf_dd, which it
-// replaces, 6.2e-8) and b' to 2e-7.  The FP64 pair exponentials e^{-l t} come from a table on a 1/32 A grid and a
-// polynomial of the rest, |l delta| <= l / 64, of degree m, which leaves out (l / 64)^(m + 1) / (m + 1)!: 3e-11 for m = 5 up
-// to l = 3.38 A^-1 (alpha 1.5 with S 2.5) and for m = 9 up to 25.  Tables are per individual, lane-private in shared
-// memory (no bank conflicts whatever a lane's index) and rebuilt each generation (tersoff_tables).  s outside the table,
-// an individual whose n is too sharp for it (checked when it is built) or whose l is beyond the polynomial takes powf_dd
-// and exp_d.
+// b and b' come from a table per individual, polynomials of degree 6 on eighths of octaves of s (bond_table.cuh):
+// t = s - s_c is exact, so b is rounded once (5.9e-8 relative; powf_dd, which it replaces, 6.2e-8) and b' to 2e-7.  The FP64
+// pair exponentials e^{-l t} come from a table on a 1/32 A grid and a polynomial of the rest, |l delta| <= l / 64, of
+// degree m, which leaves out (l / 64)^(m + 1) / (m + 1)!: 3e-11 for m = 5 up to l = 3.38 A^-1 (alpha 1.5 with S 2.5) and for
+// m = 9 up to 25.  Tables are per individual, lane-private in shared memory (no bank conflicts whatever a lane's index)
+// and rebuilt each generation (tersoff_tables).  s outside the table, an individual whose n is too sharp for it (checked
+// when it is built) or whose l is beyond the polynomial takes powf_dd and exp_d.
 //
 // Two forms of the items, by the bounds (TersoffEvView::wide).  The plain one has m = 5 and evaluates a batch that needs
 // powf_dd a second time; where l may be above 3.38 or n above 5, m = 9, and powf_dd bond by bond: 67 configurations of up
@@ -225,7 +224,7 @@ __global__ void __launch_bounds__(kTabThreads) tersoff_tables(const JobView* __r
     for (int k = 0; k < kBondPoints; ++k) f[k] = at[k][lane];
     const BondEntry e = bond_fit(f, at[kBondPoints][lane], c, h);
     // not represented: taken as outside the table
-    ta[i * 64 + lane] = make_float4(e.ok ? e.b0 : nan, e.b0lo, e.k[0], e.k[1]);
+    ta[i * 64 + lane] = make_float4(e.ok ? e.b0 : nan, e.lo, e.k[0], e.k[1]);
     ta[i * 64 + 32 + lane] = make_float4(e.k[2], e.k[3], e.k[4], e.k[5]);
     return;
   }
@@ -303,16 +302,7 @@ __device__ __forceinline__ void ev_pairs_of(const EvLane<NT, LO>& L, const EvPai
     const unsigned i = min((unsigned)((bits >> 20) - L.tab_base), (unsigned)L.tab_n);
     const float4 k0 = L.ta[i * 64], k1 = L.ta[i * 64 + 32];
     const float t = s - __int_as_float((bits & 0xfff00000) | 0x00080000);
-    float pl = fmaf(k1.w, t, k1.z), d = fmaf(k1.w, t, pl);
-    pl = fmaf(pl, t, k1.y);
-    d = fmaf(d, t, pl);
-    pl = fmaf(pl, t, k1.x);
-    d = fmaf(d, t, pl);
-    pl = fmaf(pl, t, k0.w);
-    d = fmaf(d, t, pl);
-    pl = fmaf(pl, t, k0.z);
-    db[u][h] = fmaf(d, t, pl);
-    bo[u][h] = k0.x + fmaf(pl, t, k0.y);
+    bond_eval(k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w, t, bo[u][h], db[u][h]);
   };
   if constexpr (WIDE) {
     auto s_of = [&](int u, int h) { return (float)fma(L.dh, fma(L.dh, q[u].C[h], q[u].B[h]), q[u].A[h]); };
