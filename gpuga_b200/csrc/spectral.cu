@@ -722,27 +722,26 @@ __global__ void __launch_bounds__(coef_threads(NMAX)) spectral_coefs(const JobVi
       judge(kAcceptNN / kTolNN);
     }
   }
-  if (tid < sp.n_pieces && left[tid]) bad = 1;
+  double v = 1.0;  // this thread's linear column; the last one: the reference force
+  if (ri && tid < 13) {
+    const double* c64 = J.consts64 + p;
+    const size_t st = J.Pstride;
+    // R64_* of batched.cu: qq[3], C[3], v_rc, dv_rc, rc, self
+    const double vrc = c64[6 * st], dvrc = c64[7 * st], rc = c64[8 * st];
+    const int t = tid >> 2;
+    const double qq = tid < 12 ? c64[t * st] : 0.0;
+    if (tid == 12) v = c64[9 * st];
+    else v = (tid & 3) == 0 ? qq : ((tid & 3) == 1 ? qq * (dvrc * rc - vrc) : ((tid & 3) == 2 ? qq * dvrc : c64[(3 + t) * st]));
+  }
+  // an infinite constant times the zeros of a triangle would be NaN where the sum over pairs is infinite
+  if ((tid < sp.n_pieces && left[tid]) || !(fabs(v) <= DBL_MAX)) bad = 1;
   __syncthreads();
   const bool out = bad;
   for (int c = tid; c < sp.n_nodes; c += kCoefThreads) {
     const int q = owner[c >> 3], k = c - pieces[q].node0;
     sp.coef[coef_at(sp, p, column_of(pieces[q], k))] = !out && k < 8 * need[q] ? cf[c] : 0.0;
   }
-  if (tid < sp.n_lin) {
-    double v = 1.0;  // the last linear column: the reference force
-    if (ri && tid < 13) {
-      const double* c64 = J.consts64 + p;
-      const size_t st = J.Pstride;
-      // R64_* of batched.cu: qq[3], C[3], v_rc, dv_rc, rc, self
-      const double vrc = c64[6 * st], dvrc = c64[7 * st], rc = c64[8 * st];
-      const int t = tid >> 2;
-      const double qq = tid < 12 ? c64[t * st] : 0.0;
-      if (tid == 12) v = c64[9 * st];
-      else v = (tid & 3) == 0 ? qq : ((tid & 3) == 1 ? qq * (dvrc * rc - vrc) : ((tid & 3) == 2 ? qq * dvrc : c64[(3 + t) * st]));
-    }
-    sp.coef[coef_at(sp, p, tid)] = out ? 0.0 : v;
-  }
+  if (tid < sp.n_lin) sp.coef[coef_at(sp, p, tid)] = out ? 0.0 : v;
   if (tid == 0) {
     sp.flagged[p] = out ? 1 : 0;
     unsigned long long w = 0;
