@@ -246,7 +246,8 @@ __global__ void __launch_bounds__(kTabThreads) tersoff_tables(const JobView* __r
       tk[(4 * s + 2) * 32 + lane] = sqrt(2.0 * S) * A;
       tk[(4 * s + 3) * 32 + lane] = D0 / (S - 1.0);
     }
-    tk[8 * 32 + lane] = par(6 + off) - (double)v.h0;
+    // (R1's value is in the geometry, but an undefined one makes the results undefined)
+    tk[8 * 32 + lane] = par(6 + off) - (double)v.h0 + 0.0 * par(7 + off);
     ta[v.tab_n * 64 + lane] = ta[v.tab_n * 64 + 32 + lane] = make_float4(nan, nan, nan, nan);
   }
 }

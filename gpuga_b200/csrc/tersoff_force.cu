@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kFThreadsLarge, 2) tersoff_force(const JobView
       const int p = min(it.p0 + 2 * hh + half, P - 1);
       const Consts C{J.consts, J.Pstride, p};
       switch (k) {
-        case FK_MH: return -C[TC_H];
+        case FK_MH: return -C[TC_H] + 0.0f * C[TC_R1];  // (in the geometry; undefined if R1 is)
         case FK_BETA: return C[TC_BETA];
         case FK_EN: return C[TC_EN];
         case FK_MHON: return C[TC_MHON];

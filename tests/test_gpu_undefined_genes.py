@@ -5,6 +5,7 @@ import pytest
 
 from gpuga_b200 import Fitness, synth
 from tests.test_gpu_pair_expansion import _set
+from tests.test_gpu_tersoff_pairs import _cells, _targets
 
 pytestmark = pytest.mark.gpu
 
@@ -26,3 +27,12 @@ def test_infinite_dispersion():
     assert _fitness(data, kw, 40, 6, np.inf) == np.inf
     assert np.isnan(_fitness(data, kw, 40, 6, np.nan))
     assert np.isnan(_fitness(data, kw, 40, 0, np.nan))
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("nf,nc", [(4, 6), (1, 8)])
+def test_fixed_inner_radius(nf, nc, value):
+    """R1 is fixed by its bounds and belongs to the geometry of the packed force and pair-by-pair items."""
+    data = _targets(dict(_cells([64] * nc), Nc_force=nf))
+    for gene in (6, 7):
+        assert np.isnan(_fitness(data, {}, 40, gene, value)), gene
