@@ -1001,29 +1001,33 @@ __device__ __forceinline__ void nn_pairs(const float* __restrict__ wsm, int lane
   for (int u = 0; u < NP; ++u) p2[u] = with_p2 ? (float)(p2d[u] - (double)b2) : 0.f;
 }
 
-// Individual of slot `slot` of a pair item: the population's own order, or, for a job with a pair
-// expansion (spectral.cu), the list of the individuals that it left to the direct items; limit: how
-// many there are.
-__device__ __forceinline__ int pair_individual(const JobView& J, int slot, int limit) {
-  if (slot >= limit) return -1;
-  return J.sp.list ? __ldcg(J.sp.list + slot) : slot;
+// Individual of slot `slot` of a pair item (-1: none): the population's own order, or (LISTED), for a job with a pair
+// expansion (spectral.cu), the list of the individuals that it left to the direct items.
+template <bool LISTED>
+__device__ __forceinline__ int pair_individual(const JobView& J, int slot) {
+  if constexpr (!LISTED) return slot < J.P ? slot : -1;
+  if (!J.sp.list) return slot < J.P ? slot : -1;
+  return slot < __ldcg(J.sp.count) ? __ldcg(J.sp.list + slot) : -1;
 }
 
-template <int KIND, int NMAX, bool FORCE>
-__device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, const WorkItem& it, int limit,
-                                          unsigned char* smem) {
+template <int KIND, int NMAX, bool FORCE, bool LISTED>
+__device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, const WorkItem& it, unsigned char* smem) {
   const JobView& J = jobs[it.job];
   const DevView S = J.v;
-  const int Pstride = J.Pstride, nn = J.num_neurons, nv = J.num_vars;
+  const int P = J.P, Pstride = J.Pstride, nn = J.num_neurons, nv = J.num_vars;
   const NNTaper tp = J.tp;
   const float* __restrict__ weights = J.weights;
   double* __restrict__ res = J.res;
   float* __restrict__ fdump = J.fdump;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // lane -> individual (-1: none); lanes without one compute the group's first again
-  const int p = pair_individual(J, it.p0 + lane, limit);
-  const int p_first = pair_individual(J, it.p0, limit);
-  const int pl = p >= 0 ? p : p_first;
+  // lane -> individual; lanes without one compute the group's first again
+  const int p = it.p0 + lane;  // !LISTED
+  auto lane_individual = [&](int l) {
+    if constexpr (!LISTED) return it.p0 + l < P ? it.p0 + l : it.p0;
+    const int q = pair_individual<LISTED>(J, it.p0 + l);
+    return q >= 0 ? q : pair_individual<LISTED>(J, it.p0);
+  };
+  const int pl = lane_individual(lane);
   const Consts kc{J.consts, Pstride, pl};
   RIC R;
   if (KIND == 1) load_ri(kc, R);
@@ -1033,8 +1037,7 @@ __device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, cons
     __syncthreads();
     for (int t = threadIdx.x; t < nv * 32; t += blockDim.x) {
       const int m = t >> 5, l = t & 31;
-      const int pp = pair_individual(J, it.p0 + l, limit);
-      wsm[NNSmem<NMAX>::offset(m, nn, l)] = weights[(size_t)m * Pstride + (pp >= 0 ? pp : p_first)];
+      wsm[NNSmem<NMAX>::offset(m, nn, l)] = weights[(size_t)m * Pstride + lane_individual(l)];
     }
     __syncthreads();
   }
@@ -1103,7 +1106,7 @@ __device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, cons
       const double dy = F[1] - (double)S.force_ref[i + N];
       const double dz = F[2] - (double)S.force_ref[i + 2 * (size_t)N];
       acc[7] += dx * dx + dy * dy + dz * dz;
-      if (fdump && p >= 0) {
+      if (!LISTED && fdump && p < P) {  // (per-atom forces: a launch set without a pair expansion)
         const int Nf = S.N_force;
         fdump[((size_t)p * 3 + 0) * Nf + i] = (float)F[0];
         fdump[((size_t)p * 3 + 1) * Nf + i] = (float)F[1];
@@ -1286,7 +1289,8 @@ __device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, cons
       finish_atom(0, ks);
     }
   }
-  reduce_item<32>(it, p, S.Nc, acc, smem, res);  // pair items hold 32 individuals
+  // pair items hold 32 individuals
+  reduce_item<32>(it, pair_individual<LISTED>(J, it.p0 + lane), S.Nc, acc, smem, res);
 }
 
 // RI: three CTAs per SM (at most 85 registers); NN2B: two (128 registers, two pairs per weight
@@ -1295,24 +1299,34 @@ __device__ __forceinline__ void pair_item(const JobView* __restrict__ jobs, cons
 // launch; the rigid ion's go in two launches of single-kind instantiations (job_items).
 // ONLY: 0 both kinds of items (item_force), 1 force items only, 2 energy/virial items only (one
 // body, so its own register allocation).
-// A job with a pair expansion has items here for the individuals that the expansion could not
-// represent, usually none: its items beyond their number return at once, and where every job of the
-// launch has one the grid is no larger than the GPU holds, each CTA walking the items at its stride.
-template <int KIND, int NMAX, int ONLY>
+// LISTED: some job of the launch has a pair expansion.  Its items here are for the individuals that the expansion could
+// not represent, usually none: items beyond their number return at once, and where every job of the launch has one
+// the grid is no larger than the GPU holds, each CTA walking the items at its stride.  One individual costs what a group of
+// 32 does, over every configuration.  Without: the plain items, which the list's indirection slowed by 6 to 8 %
+// (registers: 10 neurons at 8 A, forces of 8 individuals, 1.92 -> 2.08 ms).
+template <int KIND, int NMAX, int ONLY, bool LISTED>
 __global__ void __launch_bounds__(kBlock, KIND == 1 ? 3 : 2) pair_batched(const JobView* __restrict__ jobs,
                                                                          const WorkItem* __restrict__ items, int count) {
   extern __shared__ __align__(16) unsigned char smem[];
-  for (int b = blockIdx.x; b < count; b += gridDim.x) {
-    const WorkItem it = items[b];
-    const JobView& J = jobs[it.job];
-    const int limit = J.sp.list ? __ldcg(J.sp.count) : J.P;
-    if (it.p0 >= limit) continue;
-    if (b != (int)blockIdx.x) __syncthreads();  // the previous item's reads of shared memory
+  auto run = [&](const WorkItem& it) {
     if (ONLY == 1 || (ONLY == 0 && item_force(it)))
-      pair_item<KIND, NMAX, true>(jobs, it, limit, smem);
+      pair_item<KIND, NMAX, true, LISTED>(jobs, it, smem);
     else
-      pair_item<KIND, NMAX, false>(jobs, it, limit, smem);
-    finish_individuals(J, threadIdx.x < 32 ? pair_individual(J, it.p0 + (int)threadIdx.x, limit) : -1, 32);
+      pair_item<KIND, NMAX, false, LISTED>(jobs, it, smem);
+  };
+  if constexpr (!LISTED) {
+    const WorkItem it = items[blockIdx.x];
+    run(it);
+    finish_item(jobs, it, 32);
+  } else {
+    for (int b = blockIdx.x; b < count; b += gridDim.x) {
+      const WorkItem it = items[b];
+      const JobView& J = jobs[it.job];
+      if (it.p0 >= (J.sp.list ? __ldcg(J.sp.count) : J.P)) continue;
+      if (b != (int)blockIdx.x) __syncthreads();  // the previous item's reads of shared memory
+      run(it);
+      finish_individuals(J, threadIdx.x < 32 ? pair_individual<LISTED>(J, it.p0 + (int)threadIdx.x) : -1, 32);
+    }
   }
 }
 
@@ -1725,13 +1739,21 @@ int set_smem(K kernel) {
   return GPUGA_OK;
 }
 
-// configure_only: raise the dynamic shared-memory limit of the launch's kernel
-// (done when a launch set is built, never inside a stream capture).
-constexpr int kFallbackGrid = 2 * 148;  // two CTAs per SM walk the direct items of jobs with a pair expansion
+// CTAs that walk the direct items of jobs with a pair expansion: two per SM.  The rigid ion's kernel would hold three; one
+// individual of 400 over 300 oxide configurations then took 1.78 ms, with two 1.48 (all 400: 5.35 against 5.9).
+int fallback_grid(int* ctas) {
+  int dev = 0, sms = 0;
+  GPUGA_CUDA(cudaGetDevice(&dev));
+  GPUGA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  *ctas = 2 * sms;
+  return GPUGA_OK;
+}
 
-int launch_one(const LaunchSet* ls, const Launch& L, cudaStream_t st, bool configure_only) {
+// configure_only: raise the dynamic shared-memory limit of the launch's kernel and size the grid that walks the direct items
+// of jobs with a pair expansion (done when a launch set is built, never inside a stream capture).
+int launch_one(const LaunchSet* ls, Launch& L, cudaStream_t st, bool configure_only) {
   const dim3 grid(L.count), block(kBlock);
-  const dim3 pgrid(L.fallback ? std::min(L.count, kFallbackGrid) : L.count);
+  const dim3 pgrid(L.fallback ? std::min(L.count, L.grid) : L.count);
   const WorkItem* items = ls->d_items + L.first;
   if (L.packed) return tersoff_force_launch(ls->d_jobs, items, L.count, L.smem, L.nmax, L.lo, configure_only, st);
   if (L.expansion && L.kind == 0)
@@ -1754,13 +1776,18 @@ int launch_one(const LaunchSet* ls, const Launch& L, cudaStream_t st, bool confi
   do {                                                                                \
     if (L.nmax == 2) GPUGA_TERSOFF1(ZC, 2); else GPUGA_TERSOFF1(ZC, 1);               \
   } while (0)
-#define GPUGA_PAIR1(KD, NM, ON)                                                       \
+#define GPUGA_PAIR2(KD, NM, ON, LI)                                                   \
   do {                                                                                \
     if (configure_only) {                                                             \
-      GPUGA_TRY(set_smem(pair_batched<KD, NM, ON>));                                  \
+      GPUGA_TRY(set_smem(pair_batched<KD, NM, ON, LI>));                              \
+      GPUGA_TRY(fallback_grid(&L.grid));                                              \
       break;                                                                          \
     }                                                                                 \
-    pair_batched<KD, NM, ON><<<pgrid, block, L.smem, st>>>(ls->d_jobs, items, L.count); \
+    pair_batched<KD, NM, ON, LI><<<pgrid, block, L.smem, st>>>(ls->d_jobs, items, L.count); \
+  } while (0)
+#define GPUGA_PAIR1(KD, NM, ON)                                                       \
+  do {                                                                                \
+    if (L.listed) GPUGA_PAIR2(KD, NM, ON, true); else GPUGA_PAIR2(KD, NM, ON, false); \
   } while (0)
 #define GPUGA_PAIR(KD, NM) GPUGA_PAIR1(KD, NM, 0)
   if (L.kind == 0) {
@@ -1782,6 +1809,7 @@ int launch_one(const LaunchSet* ls, const Launch& L, cudaStream_t st, bool confi
 #undef GPUGA_TERSOFF1
 #undef GPUGA_PAIR
 #undef GPUGA_PAIR1
+#undef GPUGA_PAIR2
   GPUGA_CUDA(cudaGetLastError());
   return GPUGA_OK;
 }
@@ -1795,6 +1823,7 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
   std::vector<int2> indmap, specmap, by_class[5], evgroups;
   ls->jobs.clear();
   bool plain_pairs[3] = {false, false, false};  // some job of the kind evaluates every pair directly
+  bool listed_pairs[3] = {false, false, false};  // some job of the kind has a pair expansion
   for (size_t j = 0; j < jobs.size(); ++j) {
     Engine* e = jobs[j].first;
     Plan* plan = jobs[j].second;
@@ -1829,6 +1858,7 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
       plan->gscratch_floats = need;
     }
     ls->jobs.push_back(make_job_view(e, plan));
+    if (ls->direct) ls->jobs.back().sp = SpecView{};
     if (only) ls->jobs.back().ev = TersoffEvView{};  // a partial set has no tables
     if (targets) {  // the job's population / fitness live elsewhere (a device GA's buffers)
       ls->jobs.back().pop = (*targets)[j].first;
@@ -1838,8 +1868,9 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
     if (plan->ev.pairs && !only) {
       for (int g = 0; g < (plan->P + 31) / 32; ++g) evgroups.push_back(make_int2((int)j, g));
     }
-    if (plan->sp.M) {
+    if (ls->jobs.back().sp.M) {
       for (int p = 0; p < plan->P; ++p) by_class[spectral_class(e->d)].push_back(make_int2((int)j, p));
+      listed_pairs[is_ri_type(e->d.potential_type) ? 1 : 2] = true;
     } else if (e->d.potential_type != 1 && e->d.potential_type != 2) {
       plain_pairs[is_ri_type(e->d.potential_type) ? 1 : 2] = true;
     }
@@ -1847,6 +1878,7 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
   std::vector<WorkItem> all;
   ls->launches.clear();
   for (auto& kv : groups) {
+    if (ls->direct && kv.first.kind != 0 && kv.first.expansion) continue;
     auto& v = kv.second;
     std::stable_sort(v.begin(), v.end(), [](const ItemSpec& a, const ItemSpec& b) { return a.cost > b.cost; });
     Launch L;
@@ -1857,7 +1889,8 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
     L.wide = kv.first.expansion == 4;
     L.expansion = kv.first.expansion == 1 || L.wide;
     L.packed = kv.first.expansion == 2 || kv.first.expansion == 3;
-    L.fallback = L.kind != 0 && !L.expansion && !plain_pairs[L.kind];
+    L.listed = L.kind != 0 && !L.expansion && listed_pairs[L.kind];
+    L.fallback = L.listed && !plain_pairs[L.kind];
     int nforce = 0;
     for (auto& t : v) nforce += item_force(t.w) ? 1 : 0;
     L.force = nforce == 0 ? 0 : (nforce == (int)v.size() ? 1 : 2);
@@ -1913,7 +1946,7 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
   ls->tev.assign(2 * ls->launches.size(), nullptr);
   for (auto& ev : ls->tev) GPUGA_CUDA(cudaEventCreate(&ev));
   ls->t_ms.assign(ls->launches.size(), 0.0);
-  for (const Launch& L : ls->launches) GPUGA_TRY(launch_one(ls, L, nullptr, true));
+  for (Launch& L : ls->launches) GPUGA_TRY(launch_one(ls, L, nullptr, true));
   return GPUGA_OK;
 }
 
@@ -1973,7 +2006,7 @@ int launchset_enqueue(LaunchSet* ls, cudaStream_t st) {
   GPUGA_TRY(launchset_collect_timing(ls));
   int turn = 0;  // 0: st, then the side streams
   for (int k = 0; k < n_launch; ++k) {
-    const Launch& L = ls->launches[k];
+    Launch& L = ls->launches[k];
     cudaStream_t s = st;
     if (!ls->timing) {
       if (L.expansion && L.kind == 0) {
@@ -2022,7 +2055,7 @@ int time_force_items(Engine* e, Plan* plan, const std::vector<char>& only, cudaS
   int s = GPUGA_OK;
   for (int r = 0; r < 4 && s == GPUGA_OK; ++r) {
     cudaEventRecord(a, st);
-    for (const Launch& L : ls.launches)
+    for (Launch& L : ls.launches)
       if (s == GPUGA_OK) s = launch_one(&ls, L, st, false);
     cudaEventRecord(b, st);
     const cudaError_t ce = cudaEventSynchronize(b);

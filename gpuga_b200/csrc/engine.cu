@@ -146,10 +146,10 @@ namespace {
 int get_plan(Engine* e, int P, Plan** out) { return plan_get(e, P, out); }
 
 // One generation from pinned host memory to pinned host memory.
-int enqueue_generation(Engine* e, Plan* plan, cudaStream_t st) {
+int enqueue_generation(Engine* e, Plan* plan, LaunchSet* ls, cudaStream_t st) {
   const size_t nbytes = sizeof(float) * (size_t)plan->P * e->d.num_vars;
   GPUGA_CUDA(cudaMemcpyAsync(plan->d_pop, plan->h_pop, nbytes, cudaMemcpyHostToDevice, st));
-  GPUGA_TRY(launchset_enqueue(plan->ls.get(), st));
+  GPUGA_TRY(launchset_enqueue(ls, st));
   GPUGA_CUDA(cudaMemcpyAsync(plan->h_fit, plan->d_fitness, sizeof(double) * plan->P, cudaMemcpyDeviceToHost, st));
   GPUGA_CUDA(cudaMemcpyAsync(plan->h_fit + plan->P, plan->d_comps, sizeof(double) * 3 * plan->P,
                              cudaMemcpyDeviceToHost, st));
@@ -160,17 +160,18 @@ int run_batched(Engine* e, int P, const float* pop01, double* fitness, double* c
   Plan* plan = nullptr;
   GPUGA_TRY(get_plan(e, P, &plan));
   cudaStream_t st = e->stream;
+  LaunchSet* ls = plan->dump && plan->direct ? plan->direct.get() : plan->ls.get();
   // the staged path reads the plan's own population / fitness buffers
-  GPUGA_TRY(launchset_retarget(plan->ls.get(), 0, plan->d_pop, plan->d_fitness,
+  GPUGA_TRY(launchset_retarget(ls, 0, plan->d_pop, plan->d_fitness,
                                plan->dump ? plan->d_fdump : nullptr, st));
   GPUGA_CUDA(cudaStreamSynchronize(st));
   memcpy(plan->h_pop, pop01, sizeof(float) * (size_t)P * e->d.num_vars);
-  const bool use_graph = e->opt.use_graph && !plan->dump && !plan->ls->timing;
+  const bool use_graph = e->opt.use_graph && !plan->dump && !ls->timing;
   if (use_graph) {
     if (!plan->graph) {
       cudaGraph_t g = nullptr;
       GPUGA_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-      int s = enqueue_generation(e, plan, st);
+      int s = enqueue_generation(e, plan, ls, st);
       cudaError_t ce = cudaStreamEndCapture(st, &g);
       if (s != GPUGA_OK) {
         if (g) cudaGraphDestroy(g);
@@ -183,7 +184,7 @@ int run_batched(Engine* e, int P, const float* pop01, double* fitness, double* c
     }
     GPUGA_CUDA(cudaGraphLaunch(plan->graph, st));
   } else {
-    GPUGA_TRY(enqueue_generation(e, plan, st));
+    GPUGA_TRY(enqueue_generation(e, plan, ls, st));
   }
   GPUGA_CUDA(cudaStreamSynchronize(st));
   memcpy(fitness, plan->h_fit, sizeof(double) * P);
@@ -243,6 +244,12 @@ int engine_batched_forces(Engine* e, int P, const float* pop01, float* forces_ou
   GPUGA_TRY(get_plan(e, P, &plan));
   const size_t n = (size_t)P * 3 * e->d.N_force;
   if (!plan->d_fdump) GPUGA_TRY(e->alloc(&plan->d_fdump, n));
+  if (plan->sp.M && !plan->direct) {
+    std::unique_ptr<LaunchSet> ls(new LaunchSet);
+    ls->direct = true;
+    GPUGA_TRY(launchset_build({{e, plan}}, ls.get()));
+    plan->direct = std::move(ls);
+  }
   std::vector<double> fit(P);
   plan->dump = true;
   int s = run_batched(e, P, pop01, fit.data(), nullptr);

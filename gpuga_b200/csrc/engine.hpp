@@ -259,7 +259,8 @@ struct Launch {
   bool expansion = false;  // items of the pair expansion (spectral.cu), Tersoff: of pairs (tersoff_ev.cu)
   bool packed = false;     // packed Tersoff force items (tersoff_force.cu)
   bool wide = false;       // Tersoff pairs: the form for sharp n and steep exponentials (tersoff_ev.cu)
-  bool fallback = false;   // RI / NN2B direct items that only take the individuals the expansion left
+  bool listed = false;     // RI / NN2B direct items: some job has a pair expansion
+  bool fallback = false;   // every job has one: only the individuals that the expansions left
   int zclass = 4;      // Tersoff register-array size
   int nmax = 0;        // NN2B register-array size; Tersoff: number of atom types
   int force = 0;       // the launch's items: 0 energy/virial, 1 force (gather pass), 2 both
@@ -270,6 +271,7 @@ struct Launch {
   double units = 0;    // (individual, atom) pairs per launch
   double flops = 0;    // algorithmic FP32 flops per launch (FMA = 2)
   double sfu = 0;      // transcendental calls per launch
+  int grid = 0;        // fallback: CTAs, at most
 };
 
 constexpr int kSideStreams = 3;
@@ -289,6 +291,7 @@ struct LaunchSet {
   int2* d_evgroups = nullptr;  // groups of 32 individuals of jobs with pair-by-pair Tersoff items -> (job, group)
   int ev_groups = 0;
   bool folds = true;           // the items fold every individual's fitness (no fitness_jobs launch)
+  bool direct = false;         // set before the build: every pair evaluated, no pair expansion (per-atom forces)
   cudaStream_t side[kSideStreams] = {};  // launches of one generation side by side
   cudaEvent_t fork = nullptr, join[kSideStreams] = {};
   bool timing = false;               // event pair around every launch (eager launches)
@@ -336,6 +339,7 @@ struct Plan {
   bool dump = false;           // pass d_fdump to the kernels (eager launches only)
   cudaGraphExec_t graph = nullptr;
   std::unique_ptr<LaunchSet> ls;
+  std::unique_ptr<LaunchSet> direct;  // per-atom forces of a set with a pair expansion
   std::vector<int8_t> tiles;   // per configuration: the force-item TileMode (empty: default rule)
   std::shared_ptr<ItemCache> items;  // the work items of this plan (launchset_build)
   double tune_ms = 0;          // host time the autotuner took

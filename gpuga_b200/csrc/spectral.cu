@@ -16,7 +16,7 @@
 // norm over a configuration is all that a generation needs of it: |X c|^2 = |R c|^2 with X = Q R, so
 // each force configuration keeps the triangle R of at most as many rows as there are columns instead
 // of its 3 rows per atom (spec_qr).  Energy/virial configurations keep their 7 rows.
-// Per-atom forces (batched_forces) come from the direct items.
+// Per-atom forces (batched_forces) come from the direct items, in a launch set of their own.
 //
 // What it replaces: the direct items evaluate the pair function per (individual, pair) -- about 50
 // instructions for an exponential pair, 2 000 for a 16-neuron network -- and were bound by instruction
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(coef_threads(NMAX)) spectral_coefs(const JobVi
   const JobView& J = jobs[jp.x];
   const SpecView& sp = J.sp;
   const int p = jp.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) bad = J.fdump ? 1 : 0;  // per-atom forces come from the direct items
+  if (tid == 0) bad = 0;
   static_assert(sizeof(SpecPiece) % sizeof(int) == 0, "copied by words");
   for (int k = tid; k < sp.n_pieces * (int)(sizeof(SpecPiece) / sizeof(int)); k += kCoefThreads)
     reinterpret_cast<int*>(pieces)[k] = reinterpret_cast<const int*>(sp.pieces)[k];
