@@ -336,6 +336,7 @@ __global__ void spec_linear_ev(int c0, int n, SpecView sp, const double* __restr
 // by a warp (x in registers, panels of 8) took 17 ms for a tile of 648 x 648, bound by the shared-memory
 // reads of V.
 constexpr int kQrThreads = 512, kQrRows = 1024, kQrPanel = 16, kQrLd = kQrRows + 4;  // + 4: other banks
+static_assert(kSpecMaxCols <= kQrRows, "a level of the factorisation has fewer rows than the one before");
 constexpr size_t kQrSmem = sizeof(double) * (kQrPanel * kQrLd + kQrThreads / 32 * kQrPanel * 8);
 __global__ void __launch_bounds__(kQrThreads, 1) spec_qr(const QrTile* __restrict__ tiles, int n, double* __restrict__ X) {
   extern __shared__ double V[];  // [panel column][row], then [warp][panel column][8]
@@ -984,6 +985,12 @@ int factor_configs(Engine* e, const SpecView& v, int c0, int c1, const NNTaper& 
     for (int k = 0; k < ts.Na[c]; ++k) where[ts.Na_sum[c] - a0 + k] = make_int2(c - c0, 3 * k);
   }
   std::vector<void*> tmp;
+  // frees a level's work space; kernels that use it may still run (cudaFree waits for them)
+  auto drop = [&](void* p) {
+    const auto it = std::find(tmp.begin(), tmp.end(), p);
+    if (it != tmp.end()) tmp.erase(it);
+    cudaFree(p);
+  };
   auto room = [&](size_t bytes) -> void* {
     void* p = nullptr;
     if (cudaMalloc(&p, std::max<size_t>(bytes, 16)) != cudaSuccess) return nullptr;
@@ -1039,6 +1046,9 @@ int factor_configs(Engine* e, const SpecView& v, int c0, int c1, const NNTaper& 
       if (!Y || !d_to) return GPUGA_ERR_OOM;
       spec_stack<<<(unsigned)tiles.size(), 256, 0, st>>>(d_tiles, d_to, n, X, Y);
       GPUGA_CUDA(cudaGetLastError());
+      drop(X);  // (with 900 columns a level is 0.9 of the one before: a large cell has dozens)
+      drop(d_tiles);
+      drop(d_to);
       X = Y;
       cfg = stacked;
       d_cfg = put(cfg);
@@ -1146,7 +1156,7 @@ int spectral_build(Engine* e) {
   for (int b = 0; b < top; ++b)
     for (SpecPiece& pc : pieces)
       if (b < pc.K / 8) pc.cb[b] = v.ncb++;
-  if (v.n_pieces == 0 || 8 * v.ncb > kSpecMaxCols) return GPUGA_OK;
+  if (v.n_pieces == 0 || 8 * v.ncb >= kSpecMaxCols) return GPUGA_OK;  // (fewer columns than a tile's rows: levels shrink)
   const int n = 8 * v.ncb, Nev = ts.Nc - ts.Nc_force;
   const int nev_items = (Nev + kSpecEvBlocks - 1) / kSpecEvBlocks;
   std::vector<long long> moff(ts.Nc_force + nev_items + 1);
