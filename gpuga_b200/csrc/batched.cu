@@ -1952,6 +1952,8 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
   for (auto& ev : ls->tev) GPUGA_CUDA(cudaEventCreate(&ev));
   ls->t_ms.assign(ls->launches.size(), 0.0);
   for (Launch& L : ls->launches) GPUGA_TRY(launch_one(ls, L, nullptr, true));
+  // The copies above and the plan's cleared buffers are on the legacy stream, for which the engines' streams do not wait.
+  GPUGA_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   return GPUGA_OK;
 }
 

@@ -613,6 +613,7 @@ int build_geometry(Engine* e) {
     cudaFree(d_cstart);
     cudaFree(d_cell_atoms);
   };
+  GPUGA_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the uploads so far: the engine's stream does not wait for them
   neighbor_scan<kMicMode, false><<<Nc, 256, 0, st>>>(N, d.Na, d.Na_sum, rc2, d.h, d.r, d.NN, nullptr, nullptr,
                                                     nullptr, d_skip);
   GPUGA_CUDA(cudaGetLastError());

@@ -1000,7 +1000,8 @@ int factor_configs(Engine* e, const SpecView& v, int c0, int c1, const NNTaper& 
   auto put = [&](const auto& src) {
     using T = typename std::remove_reference<decltype(src)>::type::value_type;
     T* p = static_cast<T*>(room(sizeof(T) * src.size()));
-    if (p && cudaMemcpy(p, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice) != cudaSuccess) return (T*)nullptr;
+    // (in the order of the kernels: the engine's stream does not wait for the legacy one)
+    if (p && cudaMemcpyAsync(p, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice, st) != cudaSuccess) return (T*)nullptr;
     return p;
   };
   auto run = [&]() -> int {
@@ -1193,7 +1194,7 @@ int spectral_build(Engine* e) {
     using T = typename std::remove_reference<decltype(src[0])>::type;
     typename std::remove_const<T>::type* p = nullptr;
     GPUGA_TRY(e->alloc(&p, std::max<size_t>(src.size(), 1)));
-    if (!src.empty()) GPUGA_CUDA(cudaMemcpy(p, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice));
+    if (!src.empty()) GPUGA_CUDA(cudaMemcpyAsync(p, src.data(), sizeof(T) * src.size(), cudaMemcpyHostToDevice, st));
     *dst = p;
     return GPUGA_OK;
   };

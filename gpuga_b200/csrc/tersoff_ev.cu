@@ -636,11 +636,12 @@ int tersoff_ev_build(Engine* e) {
     int* d_seg0 = nullptr;
     double2* d_points = nullptr;
     GPUGA_TRY(e->alloc(&d_points, points.size()));
-    GPUGA_CUDA(cudaMemcpy(d_points, points.data(), sizeof(double2) * points.size(), cudaMemcpyHostToDevice));
+    GPUGA_CUDA(cudaMemcpyAsync(d_points, points.data(), sizeof(double2) * points.size(), cudaMemcpyHostToDevice, st));
     GPUGA_TRY(e->alloc(&d_segs, segs.size()));
     GPUGA_TRY(e->alloc(&d_seg0, seg0.size()));
-    GPUGA_CUDA(cudaMemcpy(d_segs, segs.data(), sizeof(TersoffSegment) * segs.size(), cudaMemcpyHostToDevice));
-    GPUGA_CUDA(cudaMemcpy(d_seg0, seg0.data(), sizeof(int) * seg0.size(), cudaMemcpyHostToDevice));
+    GPUGA_CUDA(cudaMemcpyAsync(d_segs, segs.data(), sizeof(TersoffSegment) * segs.size(), cudaMemcpyHostToDevice, st));
+    GPUGA_CUDA(cudaMemcpyAsync(d_seg0, seg0.data(), sizeof(int) * seg0.size(), cudaMemcpyHostToDevice, st));
+    GPUGA_CUDA(cudaStreamSynchronize(st));
     // items: consecutive segments up to kEvSegPairs pairs
     e->h_ev_items.clear();
     for (int k = 0; k < (int)segs.size();) {

@@ -464,10 +464,10 @@ int tersoff_force_build(Engine* e) {
     GPUGA_TRY(e->alloc(&d_inner, (size_t)ts.Nc));
     GPUGA_TRY(e->alloc(&d_lgH, (size_t)ts.Nc));
     GPUGA_TRY(e->alloc(&d_atom, atom.size()));
-    GPUGA_CUDA(cudaMemcpy(d_base, base.data(), sizeof(int) * ts.Nc, cudaMemcpyHostToDevice));
-    GPUGA_CUDA(cudaMemcpy(d_inner, inner.data(), sizeof(int) * ts.Nc, cudaMemcpyHostToDevice));
-    GPUGA_CUDA(cudaMemcpy(d_lgH, lgH.data(), sizeof(int) * ts.Nc, cudaMemcpyHostToDevice));
-    GPUGA_CUDA(cudaMemcpy(d_atom, atom.data(), sizeof(int) * atom.size(), cudaMemcpyHostToDevice));
+    GPUGA_CUDA(cudaMemcpyAsync(d_base, base.data(), sizeof(int) * ts.Nc, cudaMemcpyHostToDevice, st));
+    GPUGA_CUDA(cudaMemcpyAsync(d_inner, inner.data(), sizeof(int) * ts.Nc, cudaMemcpyHostToDevice, st));
+    GPUGA_CUDA(cudaMemcpyAsync(d_lgH, lgH.data(), sizeof(int) * ts.Nc, cudaMemcpyHostToDevice, st));
+    GPUGA_CUDA(cudaMemcpyAsync(d_atom, atom.data(), sizeof(int) * atom.size(), cudaMemcpyHostToDevice, st));
     GPUGA_CUDA(cudaMemcpyAsync(d_place, place.data(), sizeof(int) * n, cudaMemcpyHostToDevice, st));
     GPUGA_CUDA(cudaMemcpyAsync(d_where, where.data(), sizeof(int2) * n, cudaMemcpyHostToDevice, st));
     force_geometry<<<(n + 127) / 128, 128, 0, st>>>(n, d.off, d.nbr, d.rev, d.ptype, d.g64, r1, r2, d_rank, d_place, d_where,
