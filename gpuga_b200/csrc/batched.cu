@@ -1525,10 +1525,11 @@ static bool tersoff_consts_exact(const PotentialSpec& sp, int num_types) {
 //     NN2B:    4n^2 + 13n + 10 flops + 2n tanh per pair
 // modes: per configuration the force-item tile (TileMode; empty: the default rule for all);
 // only: when given, the configurations whose items are built (the autotuner's trial launches).
-int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<ItemSpec>>& groups,
+int job_items(const Engine* e, const Plan* plan, int job, std::map<LaunchKey, std::vector<ItemSpec>>& groups,
               std::map<LaunchKey, size_t>& smem_need, size_t* gscratch_floats, const std::vector<int8_t>* modes,
               const std::vector<char>* only) {
   *gscratch_floats = 0;
+  const int P = plan->P;
   const DevSet& d = e->d;
   const TrainingSet& ts = e->ts;
   const bool tersoff = d.potential_type == 1 || d.potential_type == 2;
@@ -1595,7 +1596,7 @@ int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<I
                   e->h_zmax[c]);
         return GPUGA_ERR_UNSUPPORTED;
       }
-      if (!force && d.ev.pairs) continue;  // pair by pair, below
+      if (!force && plan->ev.pairs) continue;  // pair by pair, below
       if (force && e->h_tf[c]) {  // packed items (tersoff_force.cu); their one tile is the rule's for every tile option
         const LaunchKey key{0, 0, nmax, 0, lo ? 1 : 0, tersoff_force_large(Na) ? 3 : 2};
         smem_need[key] = std::max(smem_need[key], tersoff_force_smem(Na));
@@ -1699,7 +1700,7 @@ int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<I
           {WorkItem{c, p0, pack_G(G, staged, fbytes, global, Grule, force, once), job, gofs}, cf * cnt, (double)Na * cnt, cf * cnt, cs * cnt});
     }
   }
-  if (d.ev.pairs && !only) {
+  if (plan->ev.pairs && !only) {
     const LaunchKey key{0, 0, nmax, 0, lo ? 1 : 0, d.ev.wide ? 4 : 1};
     smem_need[key] = std::max(smem_need[key], tersoff_ev_smem(d.ev));
     for (const EvItem& x : e->h_ev_items)
@@ -1712,7 +1713,7 @@ int job_items(const Engine* e, int P, int job, std::map<LaunchKey, std::vector<I
                                (double)x.atoms * cnt, fl, 0.0});
       }
   }
-  if (d.sp.M) {
+  if (plan->sp.M) {
     // the pair expansion's items: a force configuration, or up to kSpecEvBlocks energy/virial ones, x 32
     // individuals; the direct items above then take only the individuals that it leaves to them
     // (pair_batched)
@@ -1832,7 +1833,7 @@ int launchset_build(const std::vector<std::pair<Engine*, Plan*>>& jobs, LaunchSe
     // (a pass over every atom and bond) and reused by every launch set the job joins
     if (only || !plan->items) {
       std::shared_ptr<ItemCache> cache(new ItemCache);
-      GPUGA_TRY(job_items(e, plan->P, 0, cache->groups, cache->smem_need, &cache->need, &plan->tiles, only));
+      GPUGA_TRY(job_items(e, plan, 0, cache->groups, cache->smem_need, &cache->need, &plan->tiles, only));
       if (!only) plan->items = cache;
       for (auto& kv : cache->groups)
         for (ItemSpec t : kv.second) {
@@ -2132,8 +2133,9 @@ int plan_build(Engine* e, int P, Plan** out) {
   GPUGA_TRY(e->alloc(&plan->d_fitness, (size_t)P));
   GPUGA_TRY(e->alloc(&plan->d_comps, (size_t)3 * P));
   GPUGA_TRY(e->alloc(&plan->d_fitcnt, (size_t)P));
-  if (d.sp.M) GPUGA_TRY(spectral_plan(e, plan.get()));
-  if (d.ev.pairs) GPUGA_TRY(tersoff_ev_plan(e, plan.get()));
+  Plan* q = plan.get();
+  if (d.sp.M) GPUGA_TRY(e->optional([&] { return spectral_plan(e, q); }, [&] { return q->sp.M != nullptr; }));
+  if (d.ev.pairs) GPUGA_TRY(e->optional([&] { return tersoff_ev_plan(e, q); }, [&] { return q->ev.pairs != nullptr; }));
   GPUGA_CUDA(cudaMemset(plan->d_fitcnt, 0, sizeof(int) * (size_t)P));
   GPUGA_TRY(e->alloc(&plan->d_pop, (size_t)P * d.num_vars));
   GPUGA_CUDA(cudaMallocHost(&plan->h_pop, sizeof(float) * (size_t)P * d.num_vars));

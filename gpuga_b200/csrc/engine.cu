@@ -40,6 +40,10 @@ void Engine::dfree(void* p) {
   cudaFree(p);
 }
 
+void Engine::dfree_since(size_t n) {
+  while (allocations.size() > n) dfree(allocations.back());
+}
+
 namespace {
 template <class T>
 int upload(Engine* e, T** dst, const T* src, size_t n) {

@@ -380,6 +380,17 @@ struct Engine {
   ~Engine();
   int dalloc(void** p, size_t bytes);
   void dfree(void* p);  // frees an allocation made by dalloc before the engine's end
+  void dfree_since(size_t n);  // all after the first n
+  // An evaluation that needs memory of its own, which another can stand in for: `build` allocates it; where it gives up
+  // (kept() stays false) its allocations are freed, and where the device is out of memory that is no error.
+  template <class F, class K>
+  int optional(F build, K kept) {
+    const size_t n = allocations.size();
+    const int s = build();
+    if (s == GPUGA_OK && kept()) return s;
+    dfree_since(n);
+    return s == GPUGA_ERR_OOM ? GPUGA_OK : s;
+  }
   template <class T>
   int alloc(T** p, size_t n) {
     return dalloc(reinterpret_cast<void**>(p), n * sizeof(T));
@@ -387,8 +398,8 @@ struct Engine {
 };
 
 // spectral.cu
-int spectral_build(Engine* e);                 // moments of the training set (where the expansion pays)
-int spectral_plan(Engine* e, Plan* plan);      // per-population buffers
+int spectral_build(Engine* e);                 // moments of the training set (where the expansion pays): DevSet::sp
+int spectral_plan(Engine* e, Plan* plan);      // per-population buffers: Plan::sp
 size_t spectral_bytes(const PotentialSpec& spec, const TrainingSet& ts);  // estimate
 int spectral_class(const DevSet& d);           // 0 rigid ion, 1-4 network width classes
 // Coefficients of every individual of the set, then (per launch) the items.

@@ -783,9 +783,10 @@ int build_geometry(Engine* e) {
     if (!hb.empty()) GPUGA_CUDA(cudaMemcpy(d.hb, hb.data(), sizeof(int) * hb.size(), cudaMemcpyHostToDevice));
     GPUGA_CUDA(cudaMemcpy(d.hb_off, hb_off.data(), sizeof(int) * (Nc + 1), cudaMemcpyHostToDevice));
   }
-  GPUGA_TRY(tersoff_force_build(e));
-  GPUGA_TRY(tersoff_ev_build(e));
-  return spectral_build(e);
+  GPUGA_TRY(e->optional([&] { return tersoff_force_build(e); }, [&] { return d.tf.gu != nullptr; }));
+  if (!d.tf.gu) e->h_tf.assign(Nc, 0);
+  GPUGA_TRY(e->optional([&] { return tersoff_ev_build(e); }, [&] { return d.ev.pairs != nullptr; }));
+  return e->optional([&] { return spectral_build(e); }, [&] { return d.sp.M != nullptr; });
 }
 
 }  // namespace gpuga

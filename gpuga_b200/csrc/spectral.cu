@@ -1186,10 +1186,7 @@ int spectral_build(Engine* e) {
   const size_t bytes = sizeof(double) * (size_t)(size + 64 * 32);
   if (bytes > sp.expansion_bytes) return GPUGA_OK;
   double* M = nullptr;
-  if (e->alloc(&M, bytes / sizeof(double)) != GPUGA_OK) {  // no room: the direct path needs less
-    cudaGetLastError();
-    return GPUGA_OK;
-  }
+  GPUGA_TRY(e->alloc(&M, bytes / sizeof(double)));  // (no room: the direct path needs less)
   auto up = [&](auto** dst, const auto& src) -> int {
     using T = typename std::remove_reference<decltype(src[0])>::type;
     typename std::remove_const<T>::type* p = nullptr;
@@ -1210,13 +1207,7 @@ int spectral_build(Engine* e) {
     double size = 0.0;
     do size += 24.0 * ts.Na[c1++] * n;
     while (c1 < ts.Nc_force && size + 24.0 * ts.Na[c1] * n <= kQrBatchBytes);
-    const int s = factor_configs(e, v, c0, c1, tp, nn, active, M);
-    if (s == GPUGA_ERR_OOM) {
-      cudaGetLastError();
-      e->dfree(M);
-      return GPUGA_OK;
-    }
-    GPUGA_TRY(s);
+    GPUGA_TRY(factor_configs(e, v, c0, c1, tp, nn, active, M));
     c0 = c1;
   }
   if (Nev > 0) {
@@ -1243,8 +1234,6 @@ int spectral_plan(Engine* e, Plan* plan) {
   GPUGA_TRY(e->alloc(&v.count, 2));
   GPUGA_CUDA(cudaMemset(v.coef, 0, sizeof(double) * (size_t)groups * v.ncb * 64));
   GPUGA_CUDA(cudaMemset(v.count, 0, 2 * sizeof(int)));
-  // the items write the components they own; the others stay zero
-  GPUGA_CUDA(cudaMemset(plan->d_res, 0, sizeof(double) * (size_t)P * e->d.Nc * kResK));
   plan->sp = v;
   return GPUGA_OK;
 }

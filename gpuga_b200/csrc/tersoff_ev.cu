@@ -679,7 +679,6 @@ int tersoff_ev_plan(Engine* e, Plan* plan) {
   const size_t groups = (plan->P + 31) / 32;
   GPUGA_TRY(e->alloc(&v.tables, groups * tab_bytes(v)));
   GPUGA_TRY(e->alloc(&v.part, (size_t)std::max(v.n_part, 1) * 7 * plan->Pstride));
-  GPUGA_CUDA(cudaMemset(plan->d_res, 0, sizeof(double) * (size_t)plan->P * e->d.Nc * kResK));
   plan->ev = v;
   return GPUGA_OK;
 }
