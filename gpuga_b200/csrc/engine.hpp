@@ -400,7 +400,7 @@ struct Engine {
 // spectral.cu
 int spectral_build(Engine* e);                 // moments of the training set (where the expansion pays): DevSet::sp
 int spectral_plan(Engine* e, Plan* plan);      // per-population buffers: Plan::sp
-size_t spectral_bytes(const PotentialSpec& spec, const TrainingSet& ts);  // estimate
+size_t spectral_bytes(const PotentialSpec& spec, const TrainingSet& ts, int P);  // estimate, with a plan of P individuals
 int spectral_class(const DevSet& d);           // 0 rigid ion, 1-4 network width classes
 // Coefficients of every individual of the set, then (per launch) the items.
 int spectral_coefficients(const LaunchSet* ls, cudaStream_t st);
@@ -410,13 +410,16 @@ int spectral_items_launch(const JobView* jobs, const WorkItem* items, int count,
 int tersoff_ev_build(Engine* e);
 int tersoff_ev_plan(Engine* e, Plan* plan);
 size_t tersoff_ev_smem(const TersoffEvView& v);
-size_t tersoff_ev_table_bytes(const TersoffEvView& v);
+size_t tersoff_ev_plan_bytes(const TersoffEvView& v, int P);  // of a population
+size_t tersoff_ev_bytes(double pairs, int P);                 // estimate of a configuration of so many pairs
+size_t tersoff_ev_group_bytes(int num_types);                  // most of a group of 32 individuals
 int tersoff_tables_launch(const LaunchSet* ls, cudaStream_t st);  // tables and decode
 int tersoff_ev_items_launch(const JobView* jobs, const WorkItem* items, int count, size_t smem, int num_types, bool lo,
                             bool wide, bool configure, cudaStream_t st);
 
 // tersoff_force.cu
 int tersoff_force_build(Engine* e);
+constexpr double kTersoffForceAtomBytes = 4 * 36 + 28;  // of a packed atom
 int tersoff_force_lgH(int Na);
 bool tersoff_force_large(int Na);  // in CTAs of the larger size
 size_t tersoff_force_smem(int Na);

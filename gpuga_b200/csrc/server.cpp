@@ -90,9 +90,12 @@ struct Job {
 
 // Admission estimate of a training set's device footprint: per atom ~64 B,
 // per bond ~80 B (FP64 + FP32 geometry, indices, RI terms), per three-body
-// term 4 B, with the neighbor count estimated from the cell density.
+// term 4 B (slack), with the neighbor count estimated from the cell density; Tersoff: packed force
+// atoms, the pairs of energy/virial configurations with their sums per individual and the tables of every
+// 32 individuals; pair potentials: the expansion (spectral_bytes).
 size_t estimate_bytes(const PotentialSpec& spec, const TrainingSet& ts, int P) {
-  double bonds = 0, trip = 0, force_bonds = 0;
+  const bool tersoff = spec.type == 1 || spec.type == 2;
+  double bonds = 0, trip = 0, force_bonds = 0, fast = 0;
   const double rc = spec.cutoff;
   for (int c = 0; c < ts.Nc; ++c) {
     const float* h = ts.h.data() + 18 * (size_t)c;
@@ -104,16 +107,13 @@ size_t estimate_bytes(const PotentialSpec& spec, const TrainingSet& ts, int P) {
     bonds += na * z;
     if (c < ts.Nc_force) force_bonds += na * z;
     trip += na * z * z;
+    if (tersoff) fast += c < ts.Nc_force ? kTersoffForceAtomBytes * na : (double)tersoff_ev_bytes(0.5 * na * z, P);
   }
-  const bool tersoff = spec.type == 1 || spec.type == 2;
-  double bytes = 64.0 * ts.N + 88.0 * bonds + (tersoff ? 4.0 * trip : 0.0);
+  double bytes = 64.0 * ts.N + 88.0 * bonds + (tersoff ? 4.0 * trip : 0.0) + fast;
   bytes += (double)P * ts.Nc * kResK * 8.0 + (double)P * (spec.num_vars + 40) * 8.0;
+  if (tersoff && ts.Nc > ts.Nc_force) bytes += (P + 31) / 32 * (double)tersoff_ev_group_bytes(spec.type == 2 ? 2 : 1);
   if (spec.type == 3) bytes += 4.0 * P * force_bonds;  // NN2B force items' per-pair scratch
-  if (spec.expansion_bytes) {
-    // pair expansion: moments, at most what the engine allows, and coefficients
-    const double m = (double)spectral_bytes(spec, ts);
-    bytes += std::min(m, (double)spec.expansion_bytes) + (m > 0 ? (double)P * kSpecMaxCols * 8.0 : 0.0);
-  }
+  if (spec.expansion_bytes) bytes += (double)spectral_bytes(spec, ts, P);
   return (size_t)(1.25 * bytes) + (8u << 20);
 }
 
@@ -536,8 +536,8 @@ int gpuga_server_submit_engine(gpuga_server* s, gpuga_engine* e, int population_
   j->gens_total = generations;
   j->bytes = (size_t)((double)population_size * e->e->d.Nc * kResK * 8.0 +
                       (double)population_size * (e->e->d.num_vars + 40) * 8.0 +
-                      (e->e->d.sp.M ? (double)population_size * (e->e->d.sp.ncb * 8.0 + e->e->d.sp.n_part) * 8.0
-                                    : 0.0)) + (1u << 20);
+                      (e->e->d.sp.M ? (double)population_size * (e->e->d.sp.ncb * 8.0 + e->e->d.sp.n_part) * 8.0 : 0.0) +
+                      (e->e->d.ev.pairs ? (double)tersoff_ev_plan_bytes(e->e->d.ev, population_size) : 0.0)) + (1u << 20);
   return enqueue_job(s, std::move(j), job_id);
 }
 

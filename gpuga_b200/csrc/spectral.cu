@@ -946,20 +946,49 @@ int exp_terms(double z) {
   return K;
 }
 
+// Terms of the rigid ion's pair type t for distances lo .. hi (above kSpecMaxK: no series), from the steepest exponential
+// that the bounds allow: Buckingham 1 / rho, Morse sqrt(2 S) alpha and sqrt(2 / S) alpha.
+int ri_terms(const PotentialSpec& sp, int t, double lo, double hi) {
+  const int a = 1 + 3 * t, rho = 2 + 3 * t;
+  double k = 0.0;
+  if (sp.pmin[a] != 0.0f || sp.pmax[a] != 0.0f) {
+    if (!(sp.pmin[rho] > 0.0f) || !(sp.pmax[rho] > 0.0f)) return kSpecMaxK + 8;
+    k = 1.0 / std::min(sp.pmin[rho], sp.pmax[rho]);
+  }
+  if (t == 1 && (sp.pmin[11] != 0.0f || sp.pmax[11] != 0.0f)) {
+    const double al = std::max(std::fabs(sp.pmin[12]), std::fabs(sp.pmax[12]));
+    const double s0 = std::min(sp.pmin[14], sp.pmax[14]), s1 = std::max(sp.pmin[14], sp.pmax[14]);
+    if (!(s0 > 0.0)) return kSpecMaxK + 8;
+    k = std::max(k, std::max(std::sqrt(2.0 * s1), std::sqrt(2.0 / s0)) * al);
+  }
+  const double z = k * (0.5 * (hi - lo) * 1.02 + 1e-3);
+  return z < 200.0 ? ((exp_terms(z) + 7) & ~7) + 8 : kSpecMaxK + 8;  // one more block: it must be negligible
+}
+
 }  // namespace
 
-// Rough size of the moments: columns of the pieces (rigid ion: two types of about 48 terms; NN2B: the
-// range up to the cutoff in pieces) and 16 linear ones, times the rows kept, and the work space.
-size_t spectral_bytes(const PotentialSpec& spec, const TrainingSet& ts) {
+// At most what the expansion takes for a training set and a population of P, with the work space of the factorisation: all
+// pair types as present, distances up to the cutoff.
+size_t spectral_bytes(const PotentialSpec& spec, const TrainingSet& ts, int P) {
   if (spec.type != 3 && !is_ri_type(spec.type)) return 0;
-  const double cols =
-      16.0 + (spec.type == 3 ? kNNTerms * (std::ceil(spec.cutoff / nn_piece_length(spec.num_neurons)) + 1) : 128.0);
-  double rows = 8.0 * (ts.Nc - ts.Nc_force), all = 0.0;
+  double cols = 8.0;
+  if (spec.type == 3) {
+    cols += kNNTerms * (std::ceil(spec.cutoff / nn_piece_length(spec.num_neurons)) + 1);
+  } else {
+    cols += 8.0;
+    if (spec.pmin.size() < 15 || spec.pmax.size() < 15) return 0;
+    for (int t = 0; t < 3; ++t) cols += std::min(ri_terms(spec, t, 1.0, spec.cutoff), kSpecMaxK);
+  }
+  cols = std::min(cols, (double)kSpecMaxCols);
+  double rows = 8.0 * (ts.Nc - ts.Nc_force), all = 0.0, largest = 0.0;
   for (int c = 0; c < ts.Nc_force; ++c) {
     rows += std::min(3.0 * ts.Na[c], cols) + 8.0;
-    all += 3.0 * ts.Na[c];
+    all += 24.0 * ts.Na[c] * cols;
+    largest = std::max(largest, 24.0 * ts.Na[c] * cols);
   }
-  return (size_t)(8.0 * cols * rows + std::min(16.0 * cols * all, 2.0 * kQrBatchBytes));
+  const double moments = 8.0 * cols * rows, work = 2.0 * std::min(all, std::max(largest, kQrBatchBytes));
+  const double plan = (double)((P + 31) & ~31) * 8.0 * (cols + ts.Nc_force + (ts.Nc - ts.Nc_force) / 8 + 4);
+  return (size_t)(std::min(moments, (double)spec.expansion_bytes) + work + plan);
 }
 
 int spectral_class(const DevSet& d) {
@@ -1126,22 +1155,7 @@ int spectral_build(Engine* e) {
         add(t, a, b, s + 1 < S ? b : DBL_MAX, kNNTerms);
       }
     } else {
-      // the steepest exponential that the bounds allow: Buckingham 1 / rho, Morse sqrt(2 S) alpha and
-      // sqrt(2 / S) alpha
-      const int a = 1 + 3 * t, rho = 2 + 3 * t;
-      double k = 0.0;
-      if (sp.pmin[a] != 0.0f || sp.pmax[a] != 0.0f) {
-        if (!(sp.pmin[rho] > 0.0f) || !(sp.pmax[rho] > 0.0f)) return GPUGA_OK;
-        k = 1.0 / std::min(sp.pmin[rho], sp.pmax[rho]);
-      }
-      if (t == 1 && (sp.pmin[11] != 0.0f || sp.pmax[11] != 0.0f)) {
-        const double al = std::max(std::fabs(sp.pmin[12]), std::fabs(sp.pmax[12]));
-        const double s0 = std::min(sp.pmin[14], sp.pmax[14]), s1 = std::max(sp.pmin[14], sp.pmax[14]);
-        if (!(s0 > 0.0)) return GPUGA_OK;
-        k = std::max(k, std::max(std::sqrt(2.0 * s1), std::sqrt(2.0 / s0)) * al);
-      }
-      const double z = k * (0.5 * (hi - lo) * 1.02 + 1e-3);
-      const int K = z < 200.0 ? ((exp_terms(z) + 7) & ~7) + 8 : kSpecMaxK + 8;  // one more block: it must be negligible
+      const int K = ri_terms(sp, t, lo, hi);
       if (K > kSpecMaxK) return GPUGA_OK;
       add(t, lo, hi, DBL_MAX, K);
     }

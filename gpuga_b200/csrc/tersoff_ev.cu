@@ -505,7 +505,22 @@ __global__ void __launch_bounds__(kEvThreads, 2) tersoff_ev(const JobView* __res
 size_t tersoff_ev_smem(const TersoffEvView& v) {
   return tab_bytes(v) + sizeof(double) * 7 * kEvThreads + sizeof(EvPair) * kEvW * 2 * kEvBatch;
 }
-size_t tersoff_ev_table_bytes(const TersoffEvView& v) { return tab_bytes(v); }
+size_t tersoff_ev_plan_bytes(const TersoffEvView& v, int P) {
+  const size_t groups = ((size_t)P + 31) / 32;
+  return groups * tab_bytes(v) + sizeof(double) * 7 * std::max(v.n_part, 1) * groups * 32;
+}
+size_t tersoff_ev_group_bytes(int num_types) {
+  TersoffEvView v{};
+  v.tab_n = kTabMax;
+  v.exp_n = kExpMax;
+  v.n_exp = 2 * num_types;
+  return tab_bytes(v);
+}
+size_t tersoff_ev_bytes(double pairs, int P) {
+  const double segments = std::ceil(pairs / kEvSegPairs);
+  return (size_t)((sizeof(EvPair) + 4 * sizeof(float4)) * (pairs + kEvBatch * segments) + sizeof(TersoffSegment) * segments +
+                  (segments > 1 ? sizeof(double) * 7 * segments * ((P + 31) & ~31) : 0.0));
+}
 
 int tersoff_ev_build(Engine* e) {
   DevSet& d = e->d;
