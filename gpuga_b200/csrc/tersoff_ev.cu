@@ -568,10 +568,9 @@ int tersoff_ev_build(Engine* e) {
     double dmin = 1e300, dmax = 0.0;
     for (int a = 0; a < na; ++a) {
       start[a + 1] = start[a] + count[a];
-      if (count[a]) {
-        dmin = std::min(dmin, range[1 + a].x);
-        dmax = std::max(dmax, range[1 + a].y);
-      }
+      // (every atom's, also of those without a pair of their own: a bond without its reverse sets the largest)
+      dmin = std::min(dmin, range[1 + a].x);
+      dmax = std::max(dmax, range[1 + a].y);
     }
     if (start[na] == 0 || !(dmax < 2000.0)) return GPUGA_OK;  // (EvPair::code has 16 bits for the grid point)
     // A configuration's fixed costs (two CTA barriers and the fold over the warps) outweigh its pairs below about 64:
