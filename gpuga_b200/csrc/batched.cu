@@ -1740,27 +1740,27 @@ int set_smem(K kernel) {
   return GPUGA_OK;
 }
 
-// CTAs that walk the direct items of jobs with a pair expansion: two per SM.  The rigid ion's kernel would hold three; one
-// individual of 400 over 300 oxide configurations then took 1.78 ms, with two 1.48 (all 400: 5.35 against 5.9).
-int fallback_grid(int* ctas) {
-  int dev = 0, sms = 0;
+int device_sms(int* sms) {
+  int dev = 0;
   GPUGA_CUDA(cudaGetDevice(&dev));
-  GPUGA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  *ctas = 2 * sms;
+  GPUGA_CUDA(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev));
   return GPUGA_OK;
 }
 
-// configure_only: raise the dynamic shared-memory limit of the launch's kernel and size the grid that walks the direct items
-// of jobs with a pair expansion (done when a launch set is built, never inside a stream capture).
+// configure_only: raise the dynamic shared-memory limit of the launch's kernel and read the SM count
+// (done when a launch set is built, never inside a stream capture).
 int launch_one(const LaunchSet* ls, Launch& L, cudaStream_t st, bool configure_only) {
   const dim3 grid(L.count), block(kBlock);
-  const dim3 pgrid(L.fallback ? std::min(L.count, L.grid) : L.count);
+  // Two CTAs per SM walk the direct items of jobs with a pair expansion.  The rigid ion's kernel would hold three; one
+  // individual of 400 over 300 oxide configurations then took 1.78 ms, with two 1.48 (all 400: 5.35 against 5.9).
+  const dim3 pgrid(L.fallback ? std::min(L.count, 2 * L.sms) : L.count);
   const WorkItem* items = ls->d_items + L.first;
   if (L.packed) return tersoff_force_launch(ls->d_jobs, items, L.count, L.smem, L.nmax, L.lo, configure_only, st);
   if (L.expansion && L.kind == 0)
     return tersoff_ev_items_launch(ls->d_jobs, items, L.count, L.smem, L.nmax, L.lo, L.wide, configure_only,
                                    st);
-  if (L.expansion) return configure_only ? GPUGA_OK : spectral_items_launch(ls->d_jobs, items, L.count, st);
+  if (L.expansion)
+    return configure_only ? device_sms(&L.sms) : spectral_items_launch(ls->d_jobs, items, L.count, L.sms, st);
 #define GPUGA_TERSOFF1(ZC, NT)                                                          \
   do {                                                                                  \
     if (configure_only) {                                                               \
@@ -1781,7 +1781,7 @@ int launch_one(const LaunchSet* ls, Launch& L, cudaStream_t st, bool configure_o
   do {                                                                                \
     if (configure_only) {                                                             \
       GPUGA_TRY(set_smem(pair_batched<KD, NM, ON, LI>));                              \
-      GPUGA_TRY(fallback_grid(&L.grid));                                              \
+      GPUGA_TRY(device_sms(&L.sms));                                                  \
       break;                                                                          \
     }                                                                                 \
     pair_batched<KD, NM, ON, LI><<<pgrid, block, L.smem, st>>>(ls->d_jobs, items, L.count); \

@@ -271,7 +271,7 @@ struct Launch {
   double units = 0;    // (individual, atom) pairs per launch
   double flops = 0;    // algorithmic FP32 flops per launch (FMA = 2)
   double sfu = 0;      // transcendental calls per launch
-  int grid = 0;        // fallback: CTAs, at most
+  int sms = 0;         // RI / NN2B: SMs of the device
 };
 
 constexpr int kSideStreams = 3;
@@ -404,7 +404,7 @@ size_t spectral_bytes(const PotentialSpec& spec, const TrainingSet& ts, int P); 
 int spectral_class(const DevSet& d);           // 0 rigid ion, 1-4 network width classes
 // Coefficients of every individual of the set, then (per launch) the items.
 int spectral_coefficients(const LaunchSet* ls, cudaStream_t st);
-int spectral_items_launch(const JobView* jobs, const WorkItem* items, int count, cudaStream_t st);
+int spectral_items_launch(const JobView* jobs, const WorkItem* items, int count, int sms, cudaStream_t st);
 
 // tersoff_ev.cu
 int tersoff_ev_build(Engine* e);

@@ -1268,11 +1268,11 @@ int spectral_coefficients(const LaunchSet* ls, cudaStream_t st) {
   return GPUGA_OK;
 }
 
-int spectral_items_launch(const JobView* jobs, const WorkItem* items, int count, cudaStream_t st) {
-  // Eight warps per CTA where the items do not fill the GPU (each then has half the row blocks to walk),
+int spectral_items_launch(const JobView* jobs, const WorkItem* items, int count, int sms, cudaStream_t st) {
+  // Eight warps per CTA where there are fewer than four items per SM (each warp then has half the row blocks to walk),
   // four otherwise: 68 items of 31 configurations, 10 neurons at 8 A: 88 against 101 us per generation;
   // 2119 items of the 300-configuration oxide set: 117 against 103.  The sums do not depend on it.
-  if (count < 4 * 148) spectral_items<8, 2, 2><<<count, 256, 0, st>>>(jobs, items);
+  if (count < 4 * sms) spectral_items<8, 2, 2><<<count, 256, 0, st>>>(jobs, items);
   else spectral_items<4, 2, 4><<<count, 128, 0, st>>>(jobs, items);
   GPUGA_CUDA(cudaGetLastError());
   return GPUGA_OK;
