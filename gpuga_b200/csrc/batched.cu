@@ -1706,9 +1706,9 @@ int job_items(const Engine* e, const Plan* plan, int job, std::map<LaunchKey, st
     for (const EvItem& x : e->h_ev_items)
       for (int p0 = 0; p0 < P; p0 += 32) {
         const double cnt = std::min(32, P - p0);
-        // per pair: twice s 4, b and b' 20 and 24 for the virial; pair terms 30 (44 with two exponentials), 12 more
+        // per pair: twice s 4, b and b' 24 and 24 for the virial; pair terms 30 (44 with two exponentials), 12 more
         // for the virial
-        const double fl = (lo ? 152.0 : 138.0) * x.pairs * cnt;
+        const double fl = (lo ? 160.0 : 146.0) * x.pairs * cnt;
         groups[key].push_back({WorkItem{x.seg, p0, pack_G(32, false, 0, false, 32, false), job, x.n_segs}, fl,
                                (double)x.atoms * cnt, fl, 0.0});
       }
