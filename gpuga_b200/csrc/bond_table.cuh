@@ -1,7 +1,7 @@
 // An entry of the bond-order table of tersoff_ev.cu: b(s) = (1 + (beta s)^n)^(-1/2n) and b'(s) over an interval of
-// s as one polynomial of degree 6, b = b0 + t (k0 + t (k1 + ...)), t = s - c, in eight 32-bit words.  b0 and k0 keep
-// the remainders of their rounding: the bonds of a crystal share few entries, so that the rounding of a coefficient does not
-// average out over them (six to fourteen neighbors: error of the fitness 1.9e-8 without k0's, 1.0e-8 with it).
+// s as one polynomial of degree 6, b = b0 + t (k0 + t (k1 + ...)), t = s - c, in eight 32-bit words.  b0 and k0 have the
+// remainders of their rounding beside them: bonds that share few entries do not average it out.  The evaluation that
+// uses k0's (FINE) takes three operations more.
 //
 // b' is what the polynomial is fitted to (degree 5 through six Chebyshev nodes), b its integral from the exact b(c):
 // a polynomial through values of b has an error in b' that is 36 times its own at the ends of the interval.
@@ -10,9 +10,9 @@
 // happens to be zero can hide the rest.
 //
 // Bounds for an entry that is accepted (tests/test_bond_table_cpu.py; n from 0.3 to 50): b to 7e-8 of its size, b' to
-// 2e-7 of the entry's largest, or of 1e-3 / s where that is larger.  Of that 4e-8 may be the interpolation's; the rest
-// is the rounding of the FP32 coefficients and of their evaluation.  On eighths of octaves every entry is accepted for
-// n up to 5 (interpolation: 4e-9 for n up to 3); of those with beta s between 0.05 and 8 all but 6 % at n = 8, 15 % at
+// 2e-7 of the entry's largest (FINE: 1.3e-7), or of 1e-3 / s where that is larger.  Of that 4e-8 may be the interpolation's;
+// the rest is the rounding of the FP32 coefficients and of their evaluation.  On eighths of octaves every entry is accepted
+// for n up to 5 (interpolation: 4e-9 for n up to 3); of those with beta s between 0.05 and 8 all but 6 % at n = 8, 15 % at
 // n = 12, 18 % at n = 18.
 #pragma once
 #include <cmath>
@@ -54,6 +54,7 @@ GPUGA_BT_HD float bt_float(uint32_t i) {
 }
 
 // b and b' at s = c + t.
+template <bool FINE>
 GPUGA_BT_HD void bond_eval(float b0, float lo, float k0, float k1, float k2, float k3, float k4, float k5, float t, float& b,
                            float& db) {
   float p = fmaf(k5, t, k4), d = fmaf(k5, t, p);
@@ -63,9 +64,15 @@ GPUGA_BT_HD void bond_eval(float b0, float lo, float k0, float k1, float k2, flo
   d = fmaf(d, t, p);
   p = fmaf(p, t, k1);
   d = fmaf(d, t, p);
-  p = k0 + fmaf(p, t, bt_float(bt_bits(lo) << 16));
-  db = fmaf(d, t, p);
-  b = b0 + fmaf(p, t, lo);
+  if (FINE) {
+    p = fmaf(p, t, bt_float(bt_bits(lo) << 16));
+    db = k0 + fmaf(d, t, p);
+    b = b0 + fmaf(p, t, fmaf(k0, t, lo));
+  } else {
+    p = fmaf(p, t, k0);
+    db = fmaf(d, t, p);
+    b = b0 + fmaf(p, t, lo);
+  }
 }
 
 // b and db/ds in closed form at s = e^ls; mh = -1/(2n), lbeta = ln beta.  b = 1, b' = 0 below beta s = 1e-16

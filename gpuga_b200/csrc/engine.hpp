@@ -101,7 +101,7 @@ struct TersoffEvView {
   int tab_base, tab_n;   // b(s): first entry (top 12 bits of the FP32 s) and entries
   const double2* points; // [tab_n][9] s and ln s where the entries are evaluated (bond_table.cuh)
   int exp_base, exp_n, n_exp;  // exponentials: first grid point, grid points, tables
-  bool wide;             // the form for sharp n and steep exponentials
+  bool wide;             // the form for sharp n, steep exponentials and many bonds per atom
   int n_part, n_items;   // items per group of 32 individuals
   // per plan
   unsigned char* tables; // [individuals / 32]
@@ -258,7 +258,7 @@ struct Launch {
   int kind = 0;        // 0 Tersoff, 1 RI, 2 NN2B
   bool expansion = false;  // items of the pair expansion (spectral.cu), Tersoff: of pairs (tersoff_ev.cu)
   bool packed = false;     // packed Tersoff force items (tersoff_force.cu)
-  bool wide = false;       // Tersoff pairs: the form for sharp n and steep exponentials (tersoff_ev.cu)
+  bool wide = false;       // Tersoff pairs: the form for sharp n, steep exponentials and many bonds per atom (tersoff_ev.cu)
   bool listed = false;     // RI / NN2B direct items: some job has a pair expansion
   bool fallback = false;   // every job has one: only the individuals that the expansions left
   int zclass = 4;      // Tersoff register-array size

@@ -21,10 +21,14 @@
 // and rebuilt each generation (tersoff_tables).  s outside the table, an individual whose n is too sharp for it (checked
 // when it is built) or whose l is beyond the polynomial takes powf_dd and exp_d.
 //
-// Two forms of the items, by the bounds (TersoffEvView::wide).  The plain one has m = 5 and evaluates a batch that needs
-// powf_dd a second time; where l may be above 3.38 or n above 5, m = 9, and powf_dd bond by bond: 67 configurations of up
-// to 1000 atoms at population 333 with n from 8 to 12 and beta s around 1, 394 us a generation (530 in the plain
-// form, 458 by atom), but 202 against 192 us for n below 0.8.  A set that allows l above 25 stays with the items by atom.
+// Two forms of the items (TersoffEvView::wide).  The plain one has m = 5 and evaluates a batch that needs powf_dd a second
+// time; the other m = 9, powf_dd bond by bond, and the fine evaluation of b'.  It is taken where
+//   the bounds allow l above 3.38 (one that allows l above 25 leaves the set to the items by atom);
+//   n may be above 5: 67 configurations of up to 1000 atoms at population 333 with n from 8 to 12 and beta s around 1, 394 us
+//   a generation (530 in the plain form, 458 by atom), but 202 against 192 us for n below 0.8;
+//   atoms have more than four bonds on average: the bonds of such crystals share few entries, and the rounding of an entry's
+//   first coefficient does not average out (fitness error, geometric mean over 12 sets of 4 to 14 neighbors: plain 1.9e-8,
+//   fine 1.0e-8, by atom 1.65e-8; sets of four neighbors: below that of the items by atom in either form).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -303,7 +307,7 @@ __device__ __forceinline__ void ev_pairs_of(const EvLane<NT, LO>& L, const EvPai
     const unsigned i = min((unsigned)((bits >> 20) - L.tab_base), (unsigned)L.tab_n);
     const float4 k0 = L.ta[i * 64], k1 = L.ta[i * 64 + 32];
     const float t = s - __int_as_float((bits & 0xfff00000) | 0x00080000);
-    bond_eval(k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w, t, bo[u][h], db[u][h]);
+    bond_eval<WIDE>(k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w, t, bo[u][h], db[u][h]);
   };
   if constexpr (WIDE) {
     auto s_of = [&](int u, int h) { return (float)fma(L.dh, fma(L.dh, q[u].C[h], q[u].B[h]), q[u].A[h]); };
@@ -548,8 +552,6 @@ int tersoff_ev_build(Engine* e) {
   cudaStream_t st = e->stream;
   TersoffEvView v{};
   v.h0 = 0.5f * hlo + 0.5f * hhi;
-  // n up to which every entry of the table is accepted, and the shorter polynomial's steepest exponential
-  v.wide = steepest > kExpFlat || !(std::max(sp.pmin[4 + off], sp.pmax[4 + off]) <= 5.0f);
   int *d_count = nullptr, *d_start = nullptr, *d_place = nullptr, *d_last = nullptr, *d_slot = nullptr;
   double2* d_range = nullptr;
   std::vector<int> count(na), start(na + 1, 0);
@@ -577,6 +579,9 @@ int tersoff_ev_build(Engine* e) {
     // sets of 8-atom cells (16 pairs) took 42-66 us by atom against 55-83 here, 64-atom cells (128 pairs)
     // 52-66 against 50-66, 216-atom ones 94-103 against 51-55.
     if (start[na] < 64LL * Nev) return GPUGA_OK;
+    // the shorter polynomial's steepest exponential, n up to which every entry of the table is accepted, more than four bonds
+    // per atom (and not a few beyond the second shell)
+    v.wide = steepest > kExpFlat || !(std::max(sp.pmin[4 + off], sp.pmax[4 + off]) <= 5.0f) || 2.0 * start[na] > 4.5 * na;
     v.exp_base = (int)std::rint(dmin * 32.0);
     v.exp_n = (int)std::rint(dmax * 32.0) - v.exp_base + 1;
     if (v.exp_n > kExpMax) return GPUGA_OK;

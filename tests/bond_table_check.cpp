@@ -1,7 +1,8 @@
 // Accuracy harness for gpuga_b200/csrc/bond_table.cuh on the host (built and run by tests/test_bond_table_cpu.py): every
 // entry that is accepted, evaluated in FP32 as the items do, against b and b' in long double.
-// Arguments: n, first and last beta s.  Prints: entries, accepted, largest error of b (of its size) and of b' (of
-// the entry's largest, or of 1e-3 / s), and the largest mean error of b' over an entry (1024 points, every 20th beta).
+// Arguments: n, first and last beta s.  Prints: entries, accepted; for the plain and the fine evaluation the largest error of b
+// (of its size) and of b' (of the entry's largest, or of 1e-3 / s); and the largest mean error of the fine b' over an
+// entry (1024 points, every 20th beta).
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -29,7 +30,7 @@ static void closed(long double n, long double beta, long double s, long double& 
 int main(int argc, char** argv) {
   const double n = atof(argv[1]), z0 = atof(argv[2]), z1 = atof(argv[3]);
   long total = 0, accepted = 0;
-  double eb = 0, ed = 0, bias = 0;
+  double eb[2] = {0, 0}, ed[2] = {0, 0}, bias = 0;
   for (int k = 0; k <= 400; ++k) {
     const double beta = k == 400 ? 0.33675f : (double)(float)(0.02 * std::pow(300.0, k / 399.0));
     const double lbeta = std::log(beta), mh = -0.5 / n;
@@ -47,24 +48,30 @@ int main(int argc, char** argv) {
       ++total;
       if (!e.ok) continue;
       ++accepted;
-      long double top = 1e-3L / c, worst = 0;
+      long double top = 1e-3L / c, worst[2] = {0, 0};
+      auto eval = [&](bool fine, float s, float& b, float& d) {
+        auto f = fine ? gpuga::bond_eval<true> : gpuga::bond_eval<false>;
+        f(e.b0, e.lo, e.k[0], e.k[1], e.k[2], e.k[3], e.k[4], e.k[5], s - c, b, d);
+      };
       for (int x = 0; x <= 64; ++x) {
-        const float s = x < 64 ? from_bits((i << 20) + x * 0x4000) : std::nextafter(from_bits((i + 1) << 20), 0.0f), t = s - c;
-        float bo, d;
-        gpuga::bond_eval(e.b0, e.lo, e.k[0], e.k[1], e.k[2], e.k[3], e.k[4], e.k[5], t, bo, d);
+        const float s = x < 64 ? from_bits((i << 20) + x * 0x4000) : std::nextafter(from_bits((i + 1) << 20), 0.0f);
         long double b, db;
         closed(n, beta, s, b, db);
-        eb = std::fmax(eb, (double)(std::fabs(bo - b) / b));
-        worst = std::fmax(worst, std::fabs(d - db));
         top = std::fmax(top, std::fabs(db));
+        for (int fine = 0; fine < 2; ++fine) {
+          float bo, d;
+          eval(fine, s, bo, d);
+          eb[fine] = std::fmax(eb[fine], (double)(std::fabs(bo - b) / b));
+          worst[fine] = std::fmax(worst[fine], std::fabs(d - db));
+        }
       }
-      ed = std::fmax(ed, (double)(worst / top));
+      for (int fine = 0; fine < 2; ++fine) ed[fine] = std::fmax(ed[fine], (double)(worst[fine] / top));
       if (k % 20 > 0) continue;
       long double sum = 0;
       for (int x = 0; x < 1024; ++x) {
         const float s = from_bits((i << 20) + x * 0x400 + 0x200);
         float bo, d;
-        gpuga::bond_eval(e.b0, e.lo, e.k[0], e.k[1], e.k[2], e.k[3], e.k[4], e.k[5], s - c, bo, d);
+        eval(true, s, bo, d);
         long double b, db;
         closed(n, beta, s, b, db);
         sum += d - db;
@@ -72,6 +79,6 @@ int main(int argc, char** argv) {
       bias = std::fmax(bias, (double)(std::fabs(sum / 1024) / top));
     }
   }
-  printf("%ld %ld %.4e %.4e %.4e\n", total, accepted, eb, ed, bias);
+  printf("%ld %ld %.4e %.4e %.4e %.4e %.4e\n", total, accepted, eb[0], ed[0], eb[1], ed[1], bias);
   return 0;
 }
