@@ -48,7 +48,7 @@ namespace {
 
 constexpr int kEvThreads = 384, kEvW = kEvThreads / 32;
 constexpr int kEvBatch = 2;           // pairs that a warp takes at a time
-constexpr int kEvConsts = 10;         // doubles per individual: la, ca, lr, cr of both pair sets, dh, 1 if the table holds
+constexpr int kEvConsts = 10;         // doubles per individual: la, ca, lr, cr of both pair sets, dh (and one unused)
 constexpr int kSetBit = 1 << 16, kShellBit = 1 << 17;  // EvPair::code: pair set; a neighbor lies in R1 .. R2 (of any pair of the batch)
 constexpr int kTabMax = 80, kExpMax = 96;
 constexpr double kStep = 1.0 / 32.0;  // distance grid
@@ -265,8 +265,9 @@ __global__ void __launch_bounds__(kTabThreads) tersoff_tables(const JobView* __r
 // Bound by issue and by the shared-memory reads of the coefficients.  The 51 000 atoms x 1000 individuals of the
 // 500-configuration Si set, alone: 1.78 ms atom by atom (batched.cu), 1.10 ms bond by bond with a test per bond for
 // the table's range, the cutoff shell and the batch's end (170 instructions per bond), 0.91 ms without them (113),
-// 0.72 ms by pairs (180 instructions per pair, shared-memory wavefronts at 81 % of their peak).  Error of the 64
-// near-optimum individuals of such sets against FP64: equal to a sixth of the atom items'.
+// 0.72 ms by pairs with b' of degree 4 (180 instructions per pair, shared-memory wavefronts at 81 % of their peak), 0.75 with
+// the present one of degree 5 (wavefronts 79 %, issue slots 72 %).  Error of the 64 near-optimum individuals of such sets
+// against FP64: equal to a sixth of the atom items'.
 template <int NT, bool LO>
 struct EvLane {
   const float4* ta;   // this lane's tables

@@ -155,8 +155,8 @@ int gpuga_plan_info(gpuga_engine* e, int P, int* n_launches, double* per_launch,
  * launches, the coefficients of pair expansions and, when the items do not fold the fitness
  * (gpuga_options.fitness_fold), the fold. */
 int gpuga_plan_kernels(gpuga_engine* e, int P, int* kernels);
-/* The force-item tile of every configuration (tiles[Nc], gpuga_options.tiles codes 1-5; 0 for
- * energy/virial and non-Tersoff configurations) of the plan for population size P, and the host time
+/* The force-item tile of every configuration (tiles[Nc], gpuga_options.tiles codes 1-5, also for
+ * configurations whose items have one tile; 0 for energy/virial and non-Tersoff configurations) of the plan for population size P, and the host time
  * the autotuner spent on it. */
 int gpuga_plan_tiles(gpuga_engine* e, int P, int* tiles, int cap, double* tune_ms);
 /* Records CUDA events around every batched launch of population size P (eager launches only:
