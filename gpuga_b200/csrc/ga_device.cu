@@ -338,6 +338,7 @@ int ga_batch_build(const std::vector<DeviceGA*>& jobs, LaunchSet* ls, GABatch** 
     GPUGA_CUDA(cudaMemcpy(B->d_table[b], rows[b].data(), sizeof(GAJob) * jobs.size(), cudaMemcpyHostToDevice));
     GPUGA_CUDA(cudaEventCreateWithFlags(&B->done[b], cudaEventDisableTiming));
   }
+  GPUGA_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the copies above: the batch's stream does not wait for them
   if (B->rank_smem > 48 * 1024)
     GPUGA_CUDA(cudaFuncSetAttribute(ga_rank_jobs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)B->rank_smem));
   *out = B.release();

@@ -507,7 +507,8 @@ int upload_weights(Engine* e, const std::vector<double>& host, T** out) {
     e->p_w_bytes = need;
   }
   std::vector<T> conv(host.begin(), host.end());
-  GPUGA_CUDA(cudaMemcpy(e->p_w, conv.data(), need, cudaMemcpyHostToDevice));
+  // (on the kernels' stream: a copy on the legacy stream may still be under way when cudaMemcpy returns)
+  GPUGA_CUDA(cudaMemcpyAsync(e->p_w, conv.data(), need, cudaMemcpyHostToDevice, e->stream));
   *out = static_cast<T*>(e->p_w);
   return GPUGA_OK;
 }

@@ -224,6 +224,7 @@ int gpuga_server::setup(Job* j) {
   j->dga.reset(g);
   GPUGA_CUDA(cudaMemcpy(device_ga_population(g), j->ga.population.data(), sizeof(float) * j->ga.population.size(),
                         cudaMemcpyHostToDevice));
+  GPUGA_CUDA(cudaStreamSynchronize(cudaStreamLegacy));  // the scheduler's stream does not wait for the copy
   return GPUGA_OK;
 }
 
