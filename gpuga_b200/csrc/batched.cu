@@ -2119,6 +2119,7 @@ int tune_tiles(Engine* e, Plan* plan) {
 }  // namespace
 
 int plan_build(Engine* e, int P, Plan** out) {
+  GPUGA_TRY(build_population_paths(e));
   const DevSet& d = e->d;
   std::unique_ptr<Plan> plan(new Plan);
   plan->P = P;

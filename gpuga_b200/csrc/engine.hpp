@@ -361,6 +361,7 @@ struct Engine {
   std::vector<int> h_spec_blocks;               // pair expansion: 8 x 8 products per force configuration
   std::vector<char> h_pair_sym;                 // NN2B: per configuration, bond list symmetric
   std::map<int, std::unique_ptr<Plan>> plans;    // keyed by population size
+  bool population_paths = false;                // build_population_paths has run
   size_t device_bytes = 0;
   std::vector<void*> allocations;
   std::map<void*, size_t> allocation_bytes;
@@ -428,6 +429,9 @@ int tersoff_force_launch(const JobView* jobs, const WorkItem* items, int count, 
 
 // geometry.cu
 int build_geometry(Engine* e);
+// Packed Tersoff forces, Tersoff pairs and the pair expansion of the training set, where they apply: by the first plan, so that
+// an engine that only predicts does not pay for them.
+int build_population_paths(Engine* e);
 // FP32 neighbor rule of neighbor.cu:30-66 on reference-layout device arrays.
 int neighbor_reference_layout(int Nc, int N, int max_Na, const int* Na, const int* Na_sum, const float* r,
                               const float* h, float cutoff, int* NN, int* NL, cudaStream_t st);

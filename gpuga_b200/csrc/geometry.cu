@@ -783,10 +783,18 @@ int build_geometry(Engine* e) {
     if (!hb.empty()) GPUGA_CUDA(cudaMemcpy(d.hb, hb.data(), sizeof(int) * hb.size(), cudaMemcpyHostToDevice));
     GPUGA_CUDA(cudaMemcpy(d.hb_off, hb_off.data(), sizeof(int) * (Nc + 1), cudaMemcpyHostToDevice));
   }
+  return GPUGA_OK;
+}
+
+int build_population_paths(Engine* e) {
+  if (e->population_paths) return GPUGA_OK;
+  DevSet& d = e->d;
   GPUGA_TRY(e->optional([&] { return tersoff_force_build(e); }, [&] { return d.tf.gu != nullptr; }));
-  if (!d.tf.gu) e->h_tf.assign(Nc, 0);
+  if (!d.tf.gu) e->h_tf.assign(d.Nc, 0);
   GPUGA_TRY(e->optional([&] { return tersoff_ev_build(e); }, [&] { return d.ev.pairs != nullptr; }));
-  return e->optional([&] { return spectral_build(e); }, [&] { return d.sp.M != nullptr; });
+  GPUGA_TRY(e->optional([&] { return spectral_build(e); }, [&] { return d.sp.M != nullptr; }));
+  e->population_paths = true;
+  return GPUGA_OK;
 }
 
 }  // namespace gpuga

@@ -535,6 +535,9 @@ int gpuga_server_submit_engine(gpuga_server* s, gpuga_engine* e, int population_
   j->gp.mutation_rate = mutation_rate;
   j->gp.maximum_generation = generations;
   j->gens_total = generations;
+  GPUGA_CUDA(cudaSetDevice(s->device));
+  const int built = build_population_paths(e->e);  // what the estimate counts
+  if (built != GPUGA_OK) return built;
   j->bytes = (size_t)((double)population_size * e->e->d.Nc * kResK * 8.0 +
                       (double)population_size * (e->e->d.num_vars + 40) * 8.0 +
                       (e->e->d.sp.M ? (double)population_size * (e->e->d.sp.ncb * 8.0 + e->e->d.sp.n_part) * 8.0 : 0.0) +
